@@ -7,14 +7,109 @@
 
 namespace sesk {
 
-// Fixed-order final sum of per-CTA partial rows: out[q] = sum_b partials[b][q].
-__global__ void finalize_kernel(const double* __restrict__ partials, int nblocks, int nr, double* out) {
-    const int q = threadIdx.x;
-    if (q < nr) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += partials[(size_t)b * nr + q];
-        out[q] = s;
+// Real-space observables: per-thread FP64 sums, one partial row per CTA.
+// Points of a thread per trip: their loads (psi and V) are issued together, which
+// keeps 16-64 KB per SM in flight; the indices come from 32-bit divisions by
+// invariant integers (N < 2^31).  Bound by memory on large fields, by launch and
+// reduction latency on small ones.
+constexpr int kObsUnroll = 4;
+
+// CTAs of obs_real_kernel: one trip each until kObsBlocks (fixed by N: deterministic sums).
+inline unsigned obs_blocks(long long N, int most) {
+    const long long b = (N + 256 * kObsUnroll - 1) / (256 * kObsUnroll);
+    return (unsigned)(b < most ? b : most);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) obs_real_kernel(const cx<T>* __restrict__ psi,
+                                                       const double* __restrict__ V, ObsArgs o,
+                                                       double* partials) {
+    double acc[kRedR];
+#pragma unroll
+    for (int q = 0; q < kRedR; ++q) acc[q] = 0.0;
+    const long long stride = (long long)gridDim.x * blockDim.x * kObsUnroll;
+    for (long long first = (long long)blockIdx.x * blockDim.x * kObsUnroll + threadIdx.x; first < o.N;
+         first += stride) {
+        cx<T> pv[kObsUnroll];
+        double vv[kObsUnroll];
+#pragma unroll
+        for (int u = 0; u < kObsUnroll; ++u) {
+            const long long idx = first + (long long)u * blockDim.x;
+            const bool in = idx < o.N;
+            pv[u] = in ? psi[idx] : mk<T>((T)0, (T)0);
+            vv[u] = in ? V[idx] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kObsUnroll; ++u) {
+            const long long idx = first + (long long)u * blockDim.x;
+            if (idx >= o.N) break;
+            const uint32_t line = fdiv((uint32_t)idx, o.fnx);
+            const int i = (int)((uint32_t)idx - line * (uint32_t)o.nx);
+            const uint32_t k = fdiv(line, o.fny);
+            const int j = (int)(line - k * (uint32_t)o.ny);
+            const cx<double> p = widen(pv[u]);
+            const double w = p.x * p.x + p.y * p.y;
+            const double x = o.x0 + i * o.hx, y = o.y0 + j * o.hy, z = o.z0 + (double)(int)k * o.hz;
+            acc[0] += w;
+            acc[1] += vv[u] * w;
+            if (x >= o.xlo && x < o.xhi) acc[2] += w;
+            acc[3] += x * w;
+            acc[4] += y * w;
+            acc[5] += z * w;
+            acc[6] += x * x * w;
+            acc[7] += y * y * w;
+            acc[8] += z * z * w;
+        }
     }
+    block_reduce_store<kRedR>(acc, partials);
+}
+
+// Fixed-order final sum of the n per-CTA partial rows of NR values, by one CTA of
+// kFoldThreads threads: out[q] (and host[q], page-locked, when given) =
+// sum_b rows[b][q].  The rows are read as one array, thread t at t, t + T, ... with
+// T a multiple of NR, so that a thread stays in one column and every load is
+// coalesced; then one warp per column adds the threads' sums.  Bound by latency (one
+// thread per column reading row after row took 37 us for 592 rows; a 64^3 complex128
+// relaxation, which sums after every step, went from 56 to 35 us a step).
+constexpr int kFoldThreads = 1024;
+
+template <int NR>
+__device__ __forceinline__ void fold_rows(const double* __restrict__ rows, int n, double* out, double* host) {
+    __shared__ double red[kFoldThreads];
+    constexpr int T = kFoldThreads / NR * NR;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (t < T) {
+        const long long total = (long long)n * NR;
+        long long i = t;
+        for (; i + 3 * T < total; i += 4 * T) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] += rows[i + u * T];
+        }
+        for (; i < total; i += T) s[0] += rows[i];
+    }
+    red[t] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (warp < NR) {
+        double v = 0.0;
+        for (int j = warp + lane * NR; j < T; j += 32 * NR) v += red[j];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) {
+            out[warp] = v;
+            if (host) host[warp] = v;
+        }
+    }
+}
+
+// CTA 0: the nr_rows rows of kRedR real-space sums at `real`; CTA 1 (when launched):
+// the nk_rows rows of kRedK k-space sums at `kspace`, into out + kRedR.  host: the
+// same values in page-locked memory, valid once the stream has passed this kernel.
+__global__ void __launch_bounds__(kFoldThreads)
+    finalize_kernel(const double* __restrict__ real, int nr_rows, const double* __restrict__ kspace, int nk_rows,
+                    double* out, double* host) {
+    if (blockIdx.x == 0) fold_rows<kRedR>(real, nr_rows, out, host);
+    else fold_rows<kRedK>(kspace, nk_rows, out + kRedR, host ? host + kRedR : nullptr);
 }
 
 // ---------------------------------------------------------------------------

@@ -41,16 +41,30 @@ __global__ void __launch_bounds__(256) norm_peak_kernel(const cx<T>* __restrict_
     }
 }
 
-// out[0] = sum of the CTA sums in CTA order, out[1] = largest CTA maximum.
-__global__ void norm_peak_finalize(const double* __restrict__ partials, int nblocks, double* out) {
-    if (threadIdx.x == 0) {
-        double s = 0.0, m = 0.0;
-        for (int b = 0; b < nblocks; ++b) {
-            s += partials[2 * b];
-            m = fmax(m, partials[2 * b + 1]);
+// out[0] = sum of the CTA sums, out[1] = largest CTA maximum, by one CTA of 256
+// threads in a fixed order (one thread adding row after row took 42 us for 592
+// rows); host: the same in page-locked memory.
+__global__ void __launch_bounds__(256) norm_peak_finalize(const double* __restrict__ partials, int nblocks, double* out,
+                                                          double* host) {
+    __shared__ double ss[256], sm[256];
+    double s = 0.0, m = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += 256) {
+        s += partials[2 * b];
+        m = fmax(m, partials[2 * b + 1]);
+    }
+    ss[threadIdx.x] = s;
+    sm[threadIdx.x] = m;
+    __syncthreads();
+    for (int h = 128; h > 0; h >>= 1) {
+        if ((int)threadIdx.x < h) {
+            ss[threadIdx.x] += ss[threadIdx.x + h];
+            sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + h]);
         }
-        out[0] = s;
-        out[1] = m;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = host[0] = ss[0];
+        out[1] = host[1] = sm[0];
     }
 }
 

@@ -267,7 +267,8 @@ struct ses_solver {
     void* stwl[3] = {nullptr, nullptr, nullptr};  // FP32 remainders (lo)
     int last_axis = 0;  // highest axis with n > 1 (0 for 1D / single point)
 
-    double* partials = nullptr;
+    double* partials = nullptr;    // per-CTA rows of real-space sums
+    double* kpartials = nullptr;   // per-CTA rows of k-space sums (the reduction passes' partials)
     size_t partial_rows = 0;
     double* dsums = nullptr;
     double* hsums = nullptr;  // pinned
@@ -377,7 +378,7 @@ void release(ses_solver* h) {
     auto dfree = [&](void* p) {
         if (p) cudaFreeAsync(p, fs);
     };
-    void* ptrs[] = {h->psi, h->scratch, h->vtab, h->V, h->maskfull, h->partials, h->dsums, h->kfull, h->tw4, h->tw4l,
+    void* ptrs[] = {h->psi, h->scratch, h->vtab, h->V, h->maskfull, h->partials, h->kpartials, h->dsums, h->kfull, h->tw4, h->tw4l,
                     h->dobs, h->derr};
     for (void* p : ptrs) dfree(p);
     for (int a = 0; a < 3; ++a) {
@@ -478,7 +479,7 @@ PassArgs<T> make_args(const ses_solver* h, int axis, const void* src, void* dst)
     tb.tw4 = h->tw4;
     tb.tw4l = h->tw4l;
     tb.long_n2 = h->long1d ? h->n[1] : 0;
-    a.partials = h->partials;
+    a.partials = h->kpartials;
     return a;
 }
 
@@ -934,8 +935,9 @@ template <typename T>
 ses_status enqueue_renormalize(ses_solver* h) {
     cudaStream_t s = h->stream;
     const ObsArgs o = obs_args(h, -1e300, 1e300);
-    obs_real_kernel<T><<<kObsBlocks, 256, 0, s>>>(reinterpret_cast<const cx<T>*>(h->psi), h->V, o, h->partials);
-    finalize_kernel<<<1, 32, 0, s>>>(h->partials, kObsBlocks, kRedR, h->dsums);
+    const unsigned ob = obs_blocks(h->N, kObsBlocks);
+    obs_real_kernel<T><<<ob, 256, 0, s>>>(reinterpret_cast<const cx<T>*>(h->psi), h->V, o, h->partials);
+    finalize_kernel<<<1, kFoldThreads, 0, s>>>(h->partials, (int)ob, nullptr, 0, h->dsums, nullptr);
     const double dv = o.hx * o.hy * o.hz;
     const unsigned gb = (unsigned)std::min<long long>((h->N + 255) / 256, 148 * 16);
     renormalize_kernel<T><<<gb, 256, 0, s>>>(reinterpret_cast<cx<T>*>(h->psi), h->N, h->dsums, dv);
@@ -964,23 +966,9 @@ ObsArgs obs_args(const ses_solver* h, double xlo, double xhi) {
 template <typename T>
 ses_status enqueue_observe(ses_solver* h, double xlo, double xhi) {
     cudaStream_t s = h->stream;
-    ObsArgs o{};
-    o.N = h->N;
-    o.nx = phys_n(h, 0);
-    o.ny = phys_n(h, 1);
-    o.fnx = make_fastdiv((uint32_t)o.nx);
-    o.fny = make_fastdiv((uint32_t)o.ny);
-    o.x0 = h->box[0];
-    o.hx = (h->box[1] - h->box[0]) / phys_n(h, 0);
-    o.y0 = h->box[2];
-    o.hy = (h->box[3] - h->box[2]) / phys_n(h, 1);
-    o.z0 = h->box[4];
-    o.hz = (h->box[5] - h->box[4]) / phys_n(h, 2);
-    o.xlo = xlo;
-    o.xhi = xhi;
-    obs_real_kernel<T><<<kObsBlocks, 256, 0, s>>>(reinterpret_cast<const cx<T>*>(h->psi), h->V, o,
-                                                  h->partials);
-    finalize_kernel<<<1, 32, 0, s>>>(h->partials, kObsBlocks, kRedR, h->dsums);
+    const ObsArgs o = obs_args(h, xlo, xhi);
+    const unsigned ob = obs_blocks(h->N, kObsBlocks);
+    obs_real_kernel<T><<<ob, 256, 0, s>>>(reinterpret_cast<const cx<T>*>(h->psi), h->V, o, h->partials);
     SES_CU(cudaGetLastError());
     // k-space: phi = FFT(psi) into the scratch field, reduced in the last pass
     unsigned rows = 0;
@@ -1005,10 +993,8 @@ ses_status enqueue_observe(ses_solver* h, double xlo, double xhi) {
         SES_TRY(pass_s<T>(h, h->last_axis, h->scratch, h->scratch, SM_REDUCE, 1.0, s));
         rows = h->pp[h->last_axis].cp ? h->pp[h->last_axis].cgrid : h->pp[h->last_axis].grid;
     }
-    finalize_kernel<<<1, 32, 0, s>>>(h->partials, (int)rows, kRedK, h->dsums + kRedR);
+    finalize_kernel<<<2, kFoldThreads, 0, s>>>(h->partials, (int)ob, h->kpartials, (int)rows, h->dsums, h->hsums);
     SES_CU(cudaGetLastError());
-    SES_CU(cudaMemcpyAsync(h->hsums, h->dsums, (kRedR + kRedK) * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
     return SES_OK;
 }
 
@@ -1680,7 +1666,8 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     // complex128 halves on C64 upload/readback ((N+1)/2 * 16 B <= N*8 + 16 B)
     if ((st = dalloc(h, &h->scratch, N * h->esize + 16)) != SES_OK) return bail(st);
     h->partial_rows = rows;
-    if ((st = dalloc(h, (void**)&h->partials, rows * kRedR * sizeof(double))) != SES_OK) return bail(st);
+    if ((st = dalloc(h, (void**)&h->partials, kObsBlocks * kRedR * sizeof(double))) != SES_OK) return bail(st);
+    if ((st = dalloc(h, (void**)&h->kpartials, rows * kRedK * sizeof(double))) != SES_OK) return bail(st);
     if ((st = dalloc(h, (void**)&h->dsums, 32 * sizeof(double))) != SES_OK) return bail(st);
     static_assert(32 * sizeof(double) <= PinnedSlab::kSlot, "observable sums fit a pinned slot");
     if (!(h->hsums = static_cast<double*>(pinned_slab().get())))
@@ -3027,9 +3014,8 @@ ses_status ses_gpu_norm_and_peak(ses_handle h, double* norm, double* peak) {
     else
         norm_peak_kernel<float><<<kNormPeakBlocks, 256, 0, s>>>(reinterpret_cast<const cx<float>*>(h->psi), h->N,
                                                                 h->partials);
-    norm_peak_finalize<<<1, 32, 0, s>>>(h->partials, kNormPeakBlocks, h->dsums);
+    norm_peak_finalize<<<1, 256, 0, s>>>(h->partials, kNormPeakBlocks, h->dsums, h->hsums);
     SES_CU(cudaGetLastError());
-    SES_CU(cudaMemcpyAsync(h->hsums, h->dsums, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
     SES_TRY(wait_bounded(h, 0));
     const double dv = ((h->box[1] - h->box[0]) / phys_n(h, 0)) * ((h->box[3] - h->box[2]) / phys_n(h, 1)) *
                       ((h->box[5] - h->box[4]) / phys_n(h, 2));

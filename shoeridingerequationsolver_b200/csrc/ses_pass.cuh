@@ -506,10 +506,7 @@ __global__ void __launch_bounds__(512, 1) spass_kernel(const PassArgs<T> a) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// Real-space observables: grid-stride FP64 sums, one partial row per CTA,
-// fixed grid -> deterministic.
-// ---------------------------------------------------------------------------
+// The grid as the real-space observables see it.
 struct ObsArgs {
     long long N;
     int nx, ny;
@@ -517,35 +514,6 @@ struct ObsArgs {
     double x0, hx, y0, hy, z0, hz;
     double xlo, xhi;
 };
-
-template <typename T>
-__global__ void __launch_bounds__(256) obs_real_kernel(const cx<T>* __restrict__ psi,
-                                                       const double* __restrict__ V, ObsArgs o,
-                                                       double* partials) {
-    double acc[kRedR];
-#pragma unroll
-    for (int q = 0; q < kRedR; ++q) acc[q] = 0.0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < o.N; idx += stride) {
-        const long long line = idx / o.nx;  // 64-bit: N may exceed 2^31
-        const int i = (int)(idx - line * o.nx);
-        const long long k = line / o.ny;
-        const int j = (int)(line - k * o.ny);
-        const cx<double> p = widen(psi[idx]);
-        const double w = p.x * p.x + p.y * p.y;
-        const double x = o.x0 + i * o.hx, y = o.y0 + j * o.hy, z = o.z0 + (double)k * o.hz;
-        acc[0] += w;
-        acc[1] += V[idx] * w;
-        if (x >= o.xlo && x < o.xhi) acc[2] += w;
-        acc[3] += x * w;
-        acc[4] += y * w;
-        acc[5] += z * w;
-        acc[6] += x * x * w;
-        acc[7] += y * y * w;
-        acc[8] += z * z * w;
-    }
-    block_reduce_store<kRedR>(acc, partials);
-}
 
 template <typename S, typename D>
 __global__ void convert_kernel(const cx<S>* __restrict__ src, cx<D>* dst, long long N) {
