@@ -149,6 +149,34 @@ __global__ void build_vtab_c64(const double* __restrict__ V, cx<float>* out, lon
     }
 }
 
+// Per-axis factors cis(-theta a_q r_q) of the dipole kicks of several steps: kick s
+// (blockIdx.y) has the x, y and z factors one after the other, n0 + n1 + n2 of them --
+// a sincos per axis point and kick instead of one per cell.  delta: cis - 1
+// (complex64), without cancellation.
+constexpr int kKicks = 64;  // kicks per launch
+struct KickArgs {
+    int n[3];
+    double axis[3], origin[3], h[3];
+    double theta[kKicks];
+};
+
+__global__ void kick_factors(const KickArgs a, int delta, cx<double>* out) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int total = a.n[0] + a.n[1] + a.n[2];
+    if (i >= total) return;
+    cx<double>* o = out + (size_t)blockIdx.y * total + i;
+    int q = 0;
+    while (i >= a.n[q]) i -= a.n[q++];
+    const double ang = -a.theta[blockIdx.y] * (a.axis[q] * (a.origin[q] + i * a.h[q]));
+    double s, c;
+    if (delta) {
+        *o = cis_minus_one(ang);
+    } else {
+        sincos(ang, &s, &c);
+        *o = mk<double>(c, s);
+    }
+}
+
 // Imaginary time (imaginary_time.ixx:71-95): real weights exp(-V dtau/2) and
 // exp(-k^2 dtau/(2m)) in the tables' formats -- complex128 (w, 0), complex64
 // the delta (w - 1, 0) from expm1, so small weights-minus-one stay accurate.
@@ -209,13 +237,49 @@ __global__ void build_axis_tables(double xmin, double xmax, int n, double dt, do
     }
 }
 
+// Per-stage twiddles of a plan, forward order then reversed order: stage (R, Ns)
+// holds w^{r k n/(Ns R)} at [r Ns + k], w = e^{-2 pi i/n}, from an FP64 sincospi
+// (complex64: hi and the FP32 remainder lo).  Built here, not copied from the host:
+// a copy from pageable memory waits for the stream.
+struct StageRadices {
+    int n, nst;
+    int rad[2][kMaxStages];
+};
+
+__host__ __device__ inline int stage_entries(const StageRadices& s) {  // both orders
+    int total = 0;
+    for (int o = 0; o < 2; ++o) {
+        int Ns = 1;
+        for (int p = 0; p < s.nst; ++p) {
+            total += s.rad[o][p] * Ns;
+            Ns *= s.rad[o][p];
+        }
+    }
+    return total;
+}
+
 template <typename T>
-__global__ void build_twiddles(int n, cx<T>* tw) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) {
-        double s, c;
-        sincospi(-2.0 * (double)t / (double)n, &s, &c);
-        tw[t] = mk<T>((T)c, (T)s);
+__global__ void build_stage_twiddles(const StageRadices s, int total, cx<T>* hi, cx<T>* lo) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    int i = e;
+    for (int o = 0; o < 2; ++o) {
+        int Ns = 1;
+        for (int p = 0; p < s.nst; ++p) {
+            const int R = s.rad[o][p];
+            if (i < R * Ns) {
+                const int r = i / Ns, k = i - r * Ns;
+                const int t = r * k * (s.n / (Ns * R));  // < n
+                double sn, cs;
+                sincospi(-2.0 * (double)t / (double)s.n, &sn, &cs);
+                const cx<T> h = mk<T>((T)cs, (T)sn);
+                hi[e] = h;
+                if (lo) lo[e] = mk<T>((T)(cs - (double)h.x), (T)(sn - (double)h.y));
+                return;
+            }
+            i -= R * Ns;
+            Ns *= R;
+        }
     }
 }
 

@@ -1,6 +1,5 @@
 // Device building blocks of the split-operator step: complex arithmetic,
-// in-register radix-2/3/4/5/6/8/10/12/16/20/32 DFTs, and one Stockham autosort stage over a
-// tile of L lines held in shared memory.
+// in-register radix-2/3/4/5/6/8/9/10/12/15/16/20/32 DFTs, and the run-time plan of an axis.
 //
 // The line FFT is the forward unnormalised transform X_k = sum_n x_n e^{-2 pi i kn/N}
 // of the reference (core/src/fft.ixx:14-18).  Inverse transforms use the
@@ -13,7 +12,7 @@
 
 namespace sesk {
 
-constexpr int kMaxStages = 12;
+constexpr int kMaxStages = 6;  // of a run-time plan: any 2^a 3^b 5^c <= 4096 takes at most 5 (3125 = 5^5)
 
 template <typename T>
 struct __align__(2 * sizeof(T)) cx {
@@ -392,6 +391,58 @@ __device__ __forceinline__ void dft20(cx<T>* v) {
     }
 }
 
+// 9 = 3 x 3: three DFTs of the samples n = 3 n1 + n2, rotated by w9^{n2 k1}, then
+// three across them; output k = k1 + 3 k2.
+template <typename T>
+__device__ __forceinline__ void dft9(cx<T>* v) {
+    const CK<T> c1 = ck<T>(0.76604444311897803520);   // cos(2 pi/9)
+    const CK<T> s1 = ck<T>(0.64278760968653932632);   // sin(2 pi/9)
+    const CK<T> c2 = ck<T>(0.17364817766693034885);   // cos(4 pi/9)
+    const CK<T> s2 = ck<T>(0.98480775301220805937);   // sin(4 pi/9)
+    const CK<T> c4 = ck<T>(-0.93969262078590838405);  // cos(8 pi/9)
+    const CK<T> s4 = ck<T>(0.34202014332566873304);   // sin(8 pi/9)
+    cx<T> a[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < 3; ++n1) a[n2][n1] = v[3 * n1 + n2];
+        dft3(a[n2]);
+    }
+    a[1][1] = rotc(a[1][1], c1, s1);
+    a[1][2] = rotc(a[1][2], c2, s2);
+    a[2][1] = rotc(a[2][1], c2, s2);
+    a[2][2] = rotc(a[2][2], c4, s4);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+        cx<T> b[3] = {a[0][k1], a[1][k1], a[2][k1]};
+        dft3(b);
+#pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = b[k2];
+    }
+}
+
+// 15 = 3 x 5 by the prime-factor mapping: input n = (5 n1 + 3 n2) mod 15, output
+// k = (10 k1 + 6 k2) mod 15 (5^{-1} = 2 mod 3, 3^{-1} = 2 mod 5).
+template <typename T>
+__device__ __forceinline__ void dft15(cx<T>* v) {
+    cx<T> a[3][5];
+#pragma unroll
+    for (int n2 = 0; n2 < 5; ++n2) {
+        cx<T> c[3];
+#pragma unroll
+        for (int n1 = 0; n1 < 3; ++n1) c[n1] = v[(5 * n1 + 3 * n2) % 15];
+        dft3(c);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) a[k1][n2] = c[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+        dft5(a[k1]);
+#pragma unroll
+        for (int k2 = 0; k2 < 5; ++k2) v[(10 * k1 + 6 * k2) % 15] = a[k1][k2];
+    }
+}
+
 template <typename T, int R>
 __device__ __forceinline__ void dft(cx<T>* v) {
     if constexpr (R == 2) dft2(v);
@@ -400,147 +451,36 @@ __device__ __forceinline__ void dft(cx<T>* v) {
     else if constexpr (R == 5) dft5(v);
     else if constexpr (R == 6) dft6(v);
     else if constexpr (R == 8) dft8(v);
+    else if constexpr (R == 9) dft9(v);
     else if constexpr (R == 10) dft10(v);
     else if constexpr (R == 12) dft12(v);
+    else if constexpr (R == 15) dft15(v);
     else if constexpr (R == 16) dft16(v);
     else if constexpr (R == 20) dft20(v);
     else if constexpr (R == 32) dft32(v);
 }
 
 // ---------------------------------------------------------------------------
-// Geometry of one axis pass.  A CTA owns a tile of L lines (L a power of two)
-// of one axis of length n.  Shared-memory address of element e of tile line l
-// is l*ls + e*es: (ls, es) = (pitch, 1) for contiguous-axis tiles, (1, L) for
-// strided-axis tiles.  Butterflies are numbered line-fastest (b -> l = b % L,
-// j = b / L) so consecutive threads touch consecutive lines: conflict-free in
-// both layouts (the contiguous layout pads its pitch to an odd length).
+// Run-time plan of one axis pass (ses_line.cuh): the axis length as a product of
+// up to kMaxStages radices, in forward [0] and reversed [1] order, and the tile of
+// L lines (a power of two) that a CTA of nthreads owns.  Stage p of an order has
+// Ns = the product of the radices before it; its twiddles w^{r k n/(Ns R)} are at
+// [toff + r Ns + k] of the axis's stage-twiddle table.
 // ---------------------------------------------------------------------------
-struct Geo {
+struct LinePlan {
     int n;         // axis length
     int L;         // lines per tile
     int lshift;    // log2(L)
     int nthreads;  // threads per CTA
-    int ls, es;    // shared-memory strides
-    int nst;       // Stockham stages
-    int rad[kMaxStages];
-    int Ns[kMaxStages];        // product of the previous radices
-    int twstride[kMaxStages];  // n / (Ns * R)
-    FastDiv fNs[kMaxStages];
-    FastDiv fn;                // division by n
+    int pitch;     // contiguous tiles: elements from line to line in an exchange buffer
+    int buf;       // elements of one exchange buffer (a pass uses two in turn)
+    int rmax;      // largest radix
+    int nst;       // stages (1 for lengths that are one radix, and for length 1)
+    int rad[2][kMaxStages];
+    int Ns[2][kMaxStages];
+    int toff[2][kMaxStages];
+    FastDiv fNs[2][kMaxStages];  // division by Ns
+    FastDiv fnR[2][kMaxStages];  // division by n / R
 };
-
-// One Stockham autosort stage of radix R (E. Bainville's formulation of the
-// mixed-radix Stockham FFT): butterfly j of span Ns reads x[j + r n/R],
-// applies twiddles w^{r k n/(Ns R)} (k = j mod Ns) and writes
-// y[(j - k) R + k + r Ns].
-//
-// STREAM: source and destination are different memories (HBM -> tile or
-// tile -> HBM), so each thread runs its butterflies start to finish.
-// Otherwise the stage is in place in the tile: a thread reads all of its (up
-// to B) butterflies into registers, the CTA synchronises, then writes.
-template <typename T, int R, int B, bool STREAM, class LD, class ST>
-__device__ __forceinline__ void stage(const Geo& g, int p, const cx<T>* __restrict__ tw, LD& ld,
-                                      ST& st) {
-    const int n = g.n;
-    const int nR = n / R;
-    const int nb = g.L * nR;
-    const int Ns = g.Ns[p];
-    const int tws = g.twstride[p];
-    const FastDiv fNs = g.fNs[p];
-    if constexpr (STREAM) {
-        for (int b = (int)threadIdx.x; b < nb; b += g.nthreads) {
-            const int l = b & (g.L - 1), j = b >> g.lshift;
-            cx<T> v[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = ld(l, j + r * nR);
-            const int k = j - (int)fdiv((uint32_t)j, fNs) * Ns;
-            if (Ns > 1) {
-                const int t1 = k * tws;
-#pragma unroll
-                for (int r = 1; r < R; ++r) v[r] = v[r] * tw[r * t1];
-            }
-            dft<T, R>(v);
-            const int base = (j - k) * R + k;
-#pragma unroll
-            for (int r = 0; r < R; ++r) st(l, base + r * Ns, v[r]);
-        }
-    } else {
-        cx<T> v[B > 0 ? B : 1][R];
-#pragma unroll
-        for (int it = 0; it < B; ++it) {
-            const int b = (int)threadIdx.x + it * g.nthreads;
-            if (b < nb) {
-                const int l = b & (g.L - 1), j = b >> g.lshift;
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[it][r] = ld(l, j + r * nR);
-                if (Ns > 1) {
-                    const int k = j - (int)fdiv((uint32_t)j, fNs) * Ns;
-                    const int t1 = k * tws;
-#pragma unroll
-                    for (int r = 1; r < R; ++r) v[it][r] = v[it][r] * tw[r * t1];
-                }
-                dft<T, R>(v[it]);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int it = 0; it < B; ++it) {
-            const int b = (int)threadIdx.x + it * g.nthreads;
-            if (b < nb) {
-                const int l = b & (g.L - 1), j = b >> g.lshift;
-                const int k = j - (int)fdiv((uint32_t)j, fNs) * Ns;
-                const int base = (j - k) * R + k;
-#pragma unroll
-                for (int r = 0; r < R; ++r) st(l, base + r * Ns, v[it][r]);
-            }
-        }
-    }
-    __syncthreads();
-}
-
-template <typename T, int EPT, int R, class LD, class ST>
-__device__ __forceinline__ void stage_any(const Geo& g, int p, bool stream, const cx<T>* tw, LD& ld,
-                                          ST& st) {
-    if (stream) stage<T, R, EPT / R, true>(g, p, tw, ld, st);
-    else stage<T, R, EPT / R, false>(g, p, tw, ld, st);
-}
-
-// Full line FFT over the tile: stage 0 reads through ld0 (HBM when G_IN, the
-// tile otherwise, with any element-wise pre-op), the last stage writes through
-// stn (HBM when G_OUT, the tile otherwise, with any post-op); intermediate
-// stages stay in the shared tile.  EPT bounds the elements a thread holds in
-// an in-place stage (B = EPT / R butterflies).
-template <typename T, int EPT, bool G_IN, bool G_OUT, class LD0, class STN>
-__device__ __forceinline__ void fft_tile(const Geo& g, cx<T>* sm, const cx<T>* __restrict__ tw,
-                                         LD0& ld0, STN& stn) {
-    if (g.nst == 0) {  // length-1 axis: identity transform, element ops still apply
-        for (int l = threadIdx.x; l < g.L; l += g.nthreads) stn(l, 0, ld0(l, 0));
-        __syncthreads();
-        return;
-    }
-    for (int p = 0; p < g.nst; ++p) {
-        const bool first = p == 0, last = p == g.nst - 1;
-        // stream only when the stage's source and destination cannot alias
-        const bool stream = (first && G_IN && !last) || (last && G_OUT && !first);
-        auto ld = [&](int l, int e) -> cx<T> {
-            return first ? ld0(l, e) : sm[l * g.ls + e * g.es];
-        };
-        auto st = [&](int l, int e, cx<T> v) {
-            if (last) stn(l, e, v);
-            else sm[l * g.ls + e * g.es] = v;
-        };
-        switch (g.rad[p]) {
-            case 2: stage_any<T, EPT, 2>(g, p, stream, tw, ld, st); break;
-            case 3: stage_any<T, EPT, 3>(g, p, stream, tw, ld, st); break;
-            case 4: stage_any<T, EPT, 4>(g, p, stream, tw, ld, st); break;
-            case 5: stage_any<T, EPT, 5>(g, p, stream, tw, ld, st); break;
-            case 8: stage_any<T, EPT, 8>(g, p, stream, tw, ld, st); break;
-            case 16:
-                if constexpr (EPT >= 16) stage_any<T, EPT, 16>(g, p, stream, tw, ld, st);
-                break;
-            default: break;
-        }
-    }
-}
 
 }  // namespace sesk

@@ -23,6 +23,7 @@
 #include "ses_gpu.h"
 #include "ses_aux.cuh"
 #include "ses_engine.cuh"
+#include "ses_line.cuh"
 #include "ses_pass.cuh"
 #include "ses_plans.cuh"
 #include "ses_plane.cuh"
@@ -51,31 +52,50 @@ ses_status fail(ses_status s, const std::string& msg) {
         if (s_ != SES_OK) return s_;   \
     } while (0)
 
-constexpr int kEPT = kEPTDev;      // elements a thread holds per in-place Stockham stage
-constexpr int kMaxLog2Radix = kEPTDev >= 16 ? 4 : 3;
 constexpr int kMaxAxis = 4096;    // longest supported axis
 constexpr int kObsBlocks = 592;   // 4 x 148 SMs, fixed -> deterministic sums
 constexpr int kBodyUnroll = 8;    // interior steps per captured graph launch
+constexpr int kLineSteps = 1024;  // most steps of a 1D line in one launch (a few ms: other streams get their turn)
 
+// The radices of a run-time plan: the fewest stages, then the smallest largest radix,
+// then the largest smallest one (stages of similar width keep the same threads busy):
+// 120 = 12 x 10, 90 = 10 x 9, 1024 = 16 x 8 x 8.  Descending, so that the crossing
+// between two transforms, the longest stage, falls on the smallest radix and has the
+// most threads at work (128 = 8 x 16 left half of them waiting there).
 bool factor_radices(int n, std::vector<int>& rad) {
+    static const int kRadices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
     rad.clear();
     if (n < 1) return false;
-    int a = 0, b = 0, c = 0, m = n;
-    while (m % 2 == 0) { m /= 2; ++a; }
-    while (m % 3 == 0) { m /= 3; ++b; }
-    while (m % 5 == 0) { m /= 5; ++c; }
-    if (m != 1) return false;
-    if (a) {  // power-of-two part: fewest radix <= kMaxRadix stages, exponents balanced
-        const int p = (a + kMaxLog2Radix - 1) / kMaxLog2Radix, base = a / p, extra = a % p;
-        for (int i = 0; i < p; ++i) rad.push_back(1 << (base + (i < extra ? 1 : 0)));
+    if (n == 1) {
+        rad.push_back(1);
+        return true;
     }
-    for (int i = 0; i < b; ++i) rad.push_back(3);
-    for (int i = 0; i < c; ++i) rad.push_back(5);
-    return true;
+    std::vector<int> cur, best;
+    auto better = [&](const std::vector<int>& x, const std::vector<int>& y) {  // both descending
+        if (x.size() != y.size()) return x.size() < y.size();
+        if (x.front() != y.front()) return x.front() < y.front();
+        return x.back() > y.back();
+    };
+    auto search = [&](auto&& self, int m, int most) -> void {
+        if (m == 1) {
+            if (best.empty() || better(cur, best)) best = cur;
+            return;
+        }
+        if ((int)cur.size() == kMaxStages) return;
+        for (int r : kRadices)
+            if (r <= most && m % r == 0) {
+                cur.push_back(r);
+                self(self, m / r, r);
+                cur.pop_back();
+            }
+    };
+    search(search, n, 16);
+    rad = best;
+    return !rad.empty();
 }
 
 struct PassPlan {
-    Geo g{};
+    LinePlan g{};
     size_t smem = 0;
     unsigned grid = 0;
     long long nlines = 0;
@@ -137,47 +157,19 @@ std::vector<const PlaneEntry<T>*> plane_candidates(int nx, int ny, const PlanEnt
     return out;
 }
 
-// Per-stage twiddles of a compiled plan, forward order then reversed order:
-// stage (R, Ns) holds w^{r k N/(Ns R)} at [r*Ns + k], w = e^{-2 pi i/N}, in FP64.
-std::vector<double> stage_twiddles(int n, int r0, int r1, int r2) {
-    std::vector<double> out;
-    auto add_plan = [&](const int* rad, int cnt) {
-        int Ns = 1;
-        for (int p = 0; p < cnt; ++p) {
-            const int R = rad[p];
-            for (int r = 0; r < R; ++r)
-                for (int k = 0; k < Ns; ++k) {
-                    const long long e = ((long long)r * k * (n / (Ns * R))) % n;
-                    const double th = -2.0 * 3.14159265358979323846 * (double)e / (double)n;
-                    out.push_back(std::cos(th));
-                    out.push_back(std::sin(th));
-                }
-            Ns *= R;
-        }
-    };
-    int fwd[3], cnt = 0;
+std::vector<int> compiled_radices(int r0, int r1, int r2) {
+    std::vector<int> v;
     for (int r : {r0, r1, r2})
-        if (r > 1) fwd[cnt++] = r;
-    if (cnt == 0) fwd[cnt++] = 1;
-    int rev[3];
-    for (int i = 0; i < cnt; ++i) rev[i] = fwd[cnt - 1 - i];
-    add_plan(fwd, cnt);
-    add_plan(rev, cnt);
-    return out;
+        if (r > 1) v.push_back(r);
+    if (v.empty()) v.push_back(1);
+    return v;
 }
 
-int threads_for(int L, int n, const std::vector<int>& rad) {
-    int t = 32;
-    for (int R : rad) {
-        const int B = kEPT / R;
-        const long long nb = (long long)L * n / R;
-        t = std::max<long long>(t, (nb + B - 1) / B);
-    }
-    return (t + 31) / 32 * 32;
-}
-
-// Tile shape of one axis pass: L lines of length n, rows of >= 128/256 B for
-// coalescing, tile <= 64 KB of shared memory, <= 512 threads.
+// Run-time plan and tile of one axis pass: L lines (a power of two) of length n
+// whose widest stage fills at most kLineThreads threads and whose two exchange
+// buffers take at most 64 KB (3 CTAs per SM), L halved while the pass has fewer
+// than two CTAs per SM.  Strided tiles keep rows of 64 bytes through all of that
+// (32-byte sectors, two to a row) as far as 200 KB of buffers allow.
 bool plan_pass(int n, int esize, bool strided, long long nlines, PassPlan& pp, std::string& why) {
     std::vector<int> rad;
     if (!factor_radices(n, rad)) {
@@ -188,43 +180,45 @@ bool plan_pass(int n, int esize, bool strided, long long nlines, PassPlan& pp, s
         why = "axis length " + std::to_string(n) + " exceeds " + std::to_string(kMaxAxis);
         return false;
     }
-    int L = strided ? 256 / esize : 128 / esize;
-    while ((long long)L * n < 2048 && L < 256) L *= 2;
-    const int pitch = strided ? n : (n % 2 == 0 ? n + 1 : n);
-    while (L > 1 && (size_t)L * pitch * esize > 64 * 1024) L /= 2;
+    const int widest = n / rad.back();  // butterflies per line of the widest stage
+    const int pitch = strided ? n : line_pad(n) + 1;
+    const int least = strided ? 64 / esize : 1;
+    auto smem_of = [&](int L) { return rad.size() > 1 ? (size_t)2 * L * pitch * esize : (size_t)0; };  // exchange buffers
+    int L = 256;
+    while (L > 1 && L * widest > kLineThreads) L /= 2;
+    L = std::max(L, least);
+    while (L > least && smem_of(L) > 64 * 1024) L /= 2;
+    while (L > 1 && smem_of(L) > 200 * 1024) L /= 2;
+    while (L > least && (nlines + L - 1) / L < 2 * 148 && L / 2 * widest >= 32) L /= 2;
     while (L > 1 && L / 2 >= nlines) L /= 2;
-    int T = threads_for(L, n, rad);
-    while (T > 512 && L > 1) {
-        L /= 2;
-        T = threads_for(L, n, rad);
-    }
-    if (T > 512) {
-        why = "no tile shape for axis length " + std::to_string(n);
-        return false;
-    }
-    Geo& g = pp.g;
-    g = Geo{};
+    LinePlan& g = pp.g;
+    g = LinePlan{};
     g.n = n;
     g.L = L;
     g.lshift = 0;
     while ((1 << g.lshift) < L) ++g.lshift;
-    g.nthreads = T;
-    g.ls = strided ? 1 : pitch;
-    g.es = strided ? L : 1;
+    g.nthreads = std::min(kLineThreads, (L * widest + 31) / 32 * 32);
+    g.pitch = pitch;
+    g.buf = rad.size() > 1 ? L * pitch : 0;
+    g.rmax = rad.front();
     g.nst = (int)rad.size();
-    int Ns = 1;
-    for (int p = 0; p < g.nst; ++p) {
-        g.rad[p] = rad[p];
-        g.Ns[p] = Ns;
-        g.twstride[p] = n / (Ns * rad[p]);
-        g.fNs[p] = make_fastdiv((uint32_t)Ns);
-        Ns *= rad[p];
+    int off = 0;
+    for (int o = 0; o < 2; ++o) {
+        int Ns = 1;
+        for (int p = 0; p < g.nst; ++p) {
+            const int R = rad[o ? g.nst - 1 - p : p];
+            g.rad[o][p] = R;
+            g.Ns[o][p] = Ns;
+            g.toff[o][p] = off;
+            g.fNs[o][p] = make_fastdiv((uint32_t)Ns);
+            g.fnR[o][p] = make_fastdiv((uint32_t)(n / R));
+            off += R * Ns;
+            Ns *= R;
+        }
     }
-    g.fn = make_fastdiv((uint32_t)n);
     pp.nlines = nlines;
     pp.grid = (unsigned)((nlines + L - 1) / L);
-    pp.smem = (size_t)L * pitch * esize;
-    if (strided) pp.smem = ((pp.smem + 15) & ~(size_t)15) + (size_t)L * (16 + 16 + 8);
+    pp.smem = smem_of(L);
     return true;
 }
 
@@ -253,7 +247,6 @@ struct ses_solver {
     void* scratch = nullptr;
     void* vtab = nullptr;
     double* V = nullptr;
-    void* tw[3] = {nullptr, nullptr, nullptr};
     double* kv[3] = {nullptr, nullptr, nullptr};
     cx<double>* kd[3] = {nullptr, nullptr, nullptr};
     double* mask1[3] = {nullptr, nullptr, nullptr};
@@ -265,6 +258,9 @@ struct ses_solver {
     PassPlan pp[3];
     void* stw[3] = {nullptr, nullptr, nullptr};   // compiled-plan stage twiddles (hi)
     void* stwl[3] = {nullptr, nullptr, nullptr};  // FP32 remainders (lo)
+    // the same of the run-time plans: of axes without a compiled plan, and of x (driven steps)
+    void* ltw[3] = {nullptr, nullptr, nullptr};
+    void* ltwl[3] = {nullptr, nullptr, nullptr};
     int last_axis = 0;  // highest axis with n > 1 (0 for 1D / single point)
 
     double* partials = nullptr;    // per-CTA rows of real-space sums
@@ -302,6 +298,7 @@ struct ses_solver {
     void* kfull = nullptr;   // kinetic delta per stored k-space element
     void* tw4 = nullptr;     // W_N^{n1 k2} per element (complex64: hi part)
     void* tw4l = nullptr;    // complex64: lo part
+    cx<double>* kicks = nullptr;      // driven steps: per-axis factors of kKicks dipole kicks
     ses_observables* dobs = nullptr;  // ses_gpu_observe_async: observables finished on the device
 };
 
@@ -379,10 +376,9 @@ void release(ses_solver* h) {
         if (p) cudaFreeAsync(p, fs);
     };
     void* ptrs[] = {h->psi, h->scratch, h->vtab, h->V, h->maskfull, h->partials, h->kpartials, h->dsums, h->kfull, h->tw4, h->tw4l,
-                    h->dobs, h->derr};
+                    h->dobs, h->derr, h->kicks};
     for (void* p : ptrs) dfree(p);
     for (int a = 0; a < 3; ++a) {
-        dfree(h->tw[a]);
         dfree(h->kv[a]);
         dfree(h->kd[a]);
         dfree(h->mask1[a]);
@@ -390,6 +386,8 @@ void release(ses_solver* h) {
         dfree(h->kdf[a]);
         dfree(h->stw[a]);
         dfree(h->stwl[a]);
+        dfree(h->ltw[a]);
+        dfree(h->ltwl[a]);
     }
     pinned_slab().put(h->hsums);
     pinned_slab().put(h->herr);
@@ -401,7 +399,7 @@ void release(ses_solver* h) {
 
 template <typename K>
 void set_smem_attr(K kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 }
 
 // Bounded wait on everything queued so far on the handle's stream.
@@ -459,7 +457,6 @@ PassArgs<T> make_args(const ses_solver* h, int axis, const void* src, void* dst)
     a.fnu = make_fastdiv((uint32_t)a.nu);
     a.fny = make_fastdiv((uint32_t)ny);
     a.fnx = make_fastdiv((uint32_t)nx);
-    a.tw = reinterpret_cast<const cx<T>*>(h->tw[axis]);
     a.stw = reinterpret_cast<const cx<T>*>(h->stw[axis]);
     a.stwl = reinterpret_cast<const cx<T>*>(h->stwl[axis]);
     a.out_scale = 1.0;
@@ -483,32 +480,6 @@ PassArgs<T> make_args(const ses_solver* h, int axis, const void* src, void* dst)
     return a;
 }
 
-template <typename T>
-using XKernel = void (*)(const PassArgs<T>);
-
-template <typename T>
-XKernel<T> xkernel(int mode) {
-    switch (mode) {
-        case XM_FWD: return xpass_kernel<T, XM_FWD>;
-        case XM_INV: return xpass_kernel<T, XM_INV>;
-        case XM_START: return xpass_kernel<T, XM_START>;
-        case XM_MID: return xpass_kernel<T, XM_MID>;
-        case XM_END: return xpass_kernel<T, XM_END>;
-        case XM_1D: return xpass_kernel<T, XM_1D>;
-        default: return xpass_kernel<T, XM_REDUCE>;
-    }
-}
-
-template <typename T>
-XKernel<T> skernel(int mode) {
-    switch (mode) {
-        case SM_FWD: return spass_kernel<T, SM_FWD>;
-        case SM_INV: return spass_kernel<T, SM_INV>;
-        case SM_FUSED: return spass_kernel<T, SM_FUSED>;
-        default: return spass_kernel<T, SM_REDUCE>;
-    }
-}
-
 // Launch of a pass kernel (single-field or batched), with programmatic stream
 // serialization when the handle allows it (the kernel starts while the previous
 // kernel of the stream drains and waits in pdl_wait before touching any field).
@@ -528,10 +499,30 @@ cudaError_t launch_pass(bool pdl, void (*k)(KArgs...), unsigned grid, unsigned b
     return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);  // also recorded for cudaGetLastError
 }
 
+// A pass on the run-time plan of its axis (steps: of an XM_1D run).
+template <typename T>
+ses_status launch_line(const ses_solver* h, int axis, int mode, PassArgs<T> a, int steps, cudaStream_t s) {
+    const PassPlan& pp = h->pp[axis];
+    a.stw = reinterpret_cast<const cx<T>*>(h->ltw[axis]);
+    a.stwl = reinterpret_cast<const cx<T>*>(h->ltwl[axis]);
+    const unsigned block = (unsigned)pp.g.nthreads;
+    const size_t smem = line_args_bytes<T>() + pp.smem;
+    if (axis == 0) {
+        launch_pass(h->pdl, line_x<T>(mode, pp.g.rmax, a.tb.kick != nullptr), pp.grid, block, smem, s, a,
+                    steps);
+    } else {
+        launch_pass(h->pdl, line_s<T>(mode, pp.g.rmax), pp.grid, block, smem, s, a);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(SES_EDEVICE, std::string("pass launch: ") + cudaGetErrorString(e));
+    return SES_OK;
+}
+
 template <typename T>
 ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a, cudaStream_t s) {
     const PassPlan& pp = h->pp[axis];
-    if (pp.cp) {
+    if (!pp.cp) return launch_line<T>(h, axis, mode, a, 1, s);
+    {
         const PlanEntry<T>* e = reinterpret_cast<const PlanEntry<T>*>(pp.cp);
         const int n = h->n[axis];
         const int tl = n / e->e;
@@ -573,9 +564,6 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
             PassKernel<T> k = axis == 0 ? e->xk[mode] : e->sk[mode];
             launch_pass(h->pdl, k, pp.cgrid, pp.cblock, pp.csmem, s, a);
         }
-    } else {
-        XKernel<T> k = axis == 0 ? xkernel<T>(mode) : skernel<T>(mode);
-        launch_pass(h->pdl, k, pp.grid, (unsigned)pp.g.nthreads, pp.smem, s, a);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -588,8 +576,8 @@ struct XProg {
     int d_load = DG_NONE, d_mid = DG_NONE, d_store = DG_NONE;
     int m_load = 0, m_mid = 0, m_store = 0;
     double out_scale = 1.0;
-    double kick = 0.0;                  // dipole kick theta at this pass's potential site
-    const double* kick_axis = nullptr;  // polarization (3 doubles)
+    int steps = 1;                      // steps of an XM_1D run
+    const cx<double>* kick = nullptr;    // dipole kick at this pass's potential site: its per-axis factors
 };
 
 template <typename T>
@@ -602,19 +590,12 @@ ses_status pass_x(const ses_solver* h, const void* src, void* dst, const XProg& 
     a.m_mid = p.m_mid;
     a.m_store = p.m_store;
     a.out_scale = p.out_scale;
-    if (p.kick != 0.0) {  // driven step: the run-time-plan x pass carries the dipole kick
+    if (p.kick) {  // driven step: the run-time-plan x pass carries the dipole kick
         a.tb.kick = p.kick;
-        for (int q = 0; q < 3; ++q) {
-            a.tb.kax[q] = p.kick_axis[q];
-            a.tb.korg[q] = h->box[2 * q];
-            a.tb.kh[q] = (h->box[2 * q + 1] - h->box[2 * q]) / phys_n(h, q);
-        }
-        const PassPlan& pp = h->pp[0];
-        xkernel<T>(p.mode)<<<pp.grid, pp.g.nthreads, pp.smem, s>>>(a);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(SES_EDEVICE, std::string("driven x pass launch: ") + cudaGetErrorString(e));
-        return SES_OK;
+        return launch_line<T>(h, 0, p.mode, a, 1, s);
     }
+    // 1D lines: the whole run of steps in one launch of the run-time plan's kernel
+    if (p.mode == XM_1D && !h->long1d) return launch_line<T>(h, 0, p.mode, a, p.steps, s);
     return launch<T>(h, 0, p.mode, a, s);
 }
 
@@ -691,8 +672,11 @@ ses_status pass_long_x(const ses_solver* h, cudaStream_t s) {
 
 template <typename T>
 void set_attrs_prec() {
-    for (int m = XM_FWD; m <= XM_REDUCE; ++m) set_smem_attr(xkernel<T>(m));
-    for (int m = SM_FWD; m <= SM_REDUCE; ++m) set_smem_attr(skernel<T>(m));
+    for (int rmax : {10, 16}) {
+        for (int m = XM_FWD; m <= XM_REDUCE; ++m) set_smem_attr(line_x<T>(m, rmax, false));
+        for (int m : {XM_START, XM_MID, XM_END}) set_smem_attr(line_x<T>(m, rmax, true));
+        for (int m = SM_FWD; m <= SM_REDUCE; ++m) set_smem_attr(line_s<T>(m, rmax));
+    }
 }
 
 void init_kernel_attrs() {  // once per process; handles may be created from several threads
@@ -726,12 +710,6 @@ ses_status interior_unit(const ses_solver* h, bool mask, cudaStream_t s) {
         SES_TRY(pass_tw<T>(h, h->psi, h->psi, SM_TW_MID, p, s));
         return pass_long_x<T>(h, s);
     }
-    if (h->last_axis == 0) {  // 1D: [V M, fwd, K/N, inv]
-        p.mode = XM_1D;
-        p.d_load = DG_FULL;
-        p.m_load = mask;
-        return pass_x<T>(h, h->psi, h->psi, p, s);
-    }
     if (h->use_plane) {  // [inv y, inv x, V (M), fwd x, fwd y] [fwd z, K/N, inv z]
         p.d_mid = DG_FULL;
         p.m_mid = mask;
@@ -748,7 +726,7 @@ ses_status interior_unit(const ses_solver* h, bool mask, cudaStream_t s) {
 template <typename T>
 ses_status ensure_body(ses_solver* h, bool mask) {
     cudaGraphExec_t& ex = h->body[mask ? 1 : 0];
-    if (ex) return SES_OK;
+    if (ex || (h->last_axis == 0 && !h->long1d)) return SES_OK;  // 1D lines step in one launch, without a graph
     if (!h->cap) SES_CU(cudaStreamCreateWithFlags(&h->cap, cudaStreamNonBlocking));
     SES_CU(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
     ses_status st = SES_OK;
@@ -791,30 +769,20 @@ ses_status enqueue_steps(ses_solver* h, int S, bool mask) {
         return pass_tw<T>(h, h->psi, h->psi, SM_TW_END, last, s);
     }
     if (h->last_axis == 0) {
-        // 1D batch: [Vh] U [V M] U ... U [Vh M], each step one fused x pass
-        XProg first;
-        first.mode = XM_1D;
-        first.d_load = DG_HALF;
-        if (S == 1) {
-            first.d_store = DG_HALF;
-            first.m_store = mask;
+        // 1D: [Vh] U [V M] U ... U [Vh M], the run of steps in one launch.  Every
+        // launch ends and starts with half kicks, in the arithmetic of the full one.
+        for (int left = S; left > 0; left -= kLineSteps) {
+            XProg p;
+            p.mode = XM_1D;
+            p.steps = std::min(left, kLineSteps);
+            p.d_load = DG_HALF;
+            p.d_mid = DG_FULL;
+            p.m_mid = mask;
+            p.d_store = DG_HALF;
+            p.m_store = mask;
+            SES_TRY(pass_x<T>(h, h->psi, h->psi, p, s));
         }
-        SES_TRY(pass_x<T>(h, h->psi, h->psi, first, s));
-        if (S == 1) return SES_OK;
-        int interior = S - 2;
-        if (interior >= kBodyUnroll) SES_TRY(ensure_body<T>(h, mask));
-        while (interior >= kBodyUnroll) {
-            SES_CU(cudaGraphLaunch(h->body[mask ? 1 : 0], s));
-            interior -= kBodyUnroll;
-        }
-        for (; interior > 0; --interior) SES_TRY(interior_unit<T>(h, mask, s));
-        XProg lastp;
-        lastp.mode = XM_1D;
-        lastp.d_load = DG_FULL;
-        lastp.m_load = mask;
-        lastp.d_store = DG_HALF;
-        lastp.m_store = mask;
-        return pass_x<T>(h, h->psi, h->psi, lastp, s);
+        return SES_OK;
     }
     // 3D / 2D: [V/2, fwd x] [y, z] {[inv x, V (M), fwd x] [y, z]} ... [inv x, V/2 (M)];
     // two-sweep 3D: [V/2, fwd x, fwd y] [z] {[inv y, inv x, V (M), fwd x, fwd y] [z]} ... [inv y, inv x, V/2 (M)]
@@ -847,38 +815,43 @@ ses_status enqueue_steps(ses_solver* h, int S, bool mask) {
 // kick theta(t) = amplitude cos(omega t) dt/2; the kicks are diagonal like the
 // potential, so they ride on the x passes that apply it (the kick ending step s
 // and the one starting step s + 1 as one phase).  Direct launches: the phases
-// change every step.
+// change every step; the per-axis factors of kKicks of them are built at a time.
 template <typename T>
 ses_status enqueue_driven(ses_solver* h, int S, bool mask, const double* axis, double amp, double omega,
                           double t0) {
     cudaStream_t s = h->stream;
     const double dt = h->dt;
     auto theta = [&](double t) { return amp * std::cos(omega * t) * 0.5 * dt; };
-    XProg start;
-    start.mode = XM_START;
-    start.d_load = DG_HALF;
-    start.kick = theta(t0);
-    start.kick_axis = axis;
-    SES_TRY(pass_x<T>(h, h->psi, h->psi, start, s));
-    SES_TRY(mid_axes<T>(h, s));
-    for (int k = 1; k < S; ++k) {
-        const double t_prev = t0 + (k - 1) * dt, t = t0 + k * dt;
-        XProg mid;
-        mid.mode = XM_MID;
-        mid.d_mid = DG_FULL;
-        mid.m_mid = mask;
-        mid.kick = theta(t_prev + dt) + theta(t);
-        mid.kick_axis = axis;
-        SES_TRY(pass_x<T>(h, h->psi, h->psi, mid, s));
-        SES_TRY(mid_axes<T>(h, s));
+    const int per_kick = h->n[0] + h->n[1] + h->n[2];
+    if (!h->kicks) SES_TRY(dalloc(h, (void**)&h->kicks, (size_t)kKicks * per_kick * sizeof(cx<double>)));
+    for (int i = 0; i <= S; ++i) {  // kick i: before step i, between steps i - 1 and i, after the last
+        if (i % kKicks == 0) {
+            KickArgs a{};
+            for (int q = 0; q < 3; ++q) {
+                a.n[q] = h->n[q];
+                a.axis[q] = axis[q];
+                a.origin[q] = h->box[2 * q];
+                a.h[q] = (h->box[2 * q + 1] - h->box[2 * q]) / phys_n(h, q);
+            }
+            const int cnt = std::min(kKicks, S + 1 - i);
+            for (int k = 0; k < cnt; ++k) {
+                const double t = t0 + (i + k) * dt, t_prev = t0 + (i + k - 1) * dt;
+                a.theta[k] = (i + k > 0 ? theta(t_prev + dt) : 0.0) + (i + k < S ? theta(t) : 0.0);
+            }
+            kick_factors<<<dim3((unsigned)(per_kick + 127) / 128, (unsigned)cnt), 128, 0, s>>>(
+                a, h->prec == SES_C64 ? 1 : 0, h->kicks);
+            SES_CU(cudaGetLastError());
+        }
+        XProg p;
+        p.mode = i == 0 ? XM_START : (i < S ? XM_MID : XM_END);
+        p.kick = h->kicks + (size_t)(i % kKicks) * per_kick;
+        if (i == 0) p.d_load = DG_HALF;
+        else if (i < S) p.d_mid = DG_FULL, p.m_mid = mask;
+        else p.d_store = DG_HALF, p.m_store = mask;
+        SES_TRY(pass_x<T>(h, h->psi, h->psi, p, s));
+        if (i < S) SES_TRY(mid_axes<T>(h, s));
     }
-    XProg end;
-    end.mode = XM_END;
-    end.d_store = DG_HALF;
-    end.m_store = mask;
-    end.kick = theta(t0 + (S - 1) * dt + dt);
-    end.kick_axis = axis;
-    return pass_x<T>(h, h->psi, h->psi, end, s);
+    return SES_OK;
 }
 
 // Natural-order transform of a long 1D line x[n1 + N1 n2] (fft(std::vector<cd>&),
@@ -1472,33 +1445,46 @@ void attach_compiled_plan(ses_solver* h, int axis) {
     }
 }
 
-ses_status upload_stage_twiddles(ses_solver* h) {
+// A plan's stage twiddles on the device: complex128, or complex64 as hi + FP32 remainder.
+ses_status make_twiddles(ses_solver* h, int n, const std::vector<int>& radices, void** hi, void** lo) {
+    StageRadices sr{};
+    sr.n = n;
+    sr.nst = (int)radices.size();
+    for (int p = 0; p < sr.nst; ++p) {
+        sr.rad[0][p] = radices[p];
+        sr.rad[1][p] = radices[sr.nst - 1 - p];
+    }
+    const int total = stage_entries(sr);
+    const unsigned gb = (unsigned)(total + 127) / 128;
+    SES_TRY(dalloc(h, hi, (size_t)total * h->esize));
+    if (h->prec == SES_C128) {
+        build_stage_twiddles<double><<<gb, 128, 0, h->stream>>>(sr, total, reinterpret_cast<cx<double>*>(*hi), nullptr);
+    } else {
+        SES_TRY(dalloc(h, lo, (size_t)total * h->esize));
+        build_stage_twiddles<float><<<gb, 128, 0, h->stream>>>(sr, total, reinterpret_cast<cx<float>*>(*hi),
+                                                               reinterpret_cast<cx<float>*>(*lo));
+    }
+    SES_CU(cudaGetLastError());
+    return SES_OK;
+}
+
+ses_status make_stage_twiddles(ses_solver* h) {
     for (int a = 0; a < 3; ++a) {
         const PassPlan& pp = h->pp[a];
-        if (!pp.cp) continue;
-        int r0, r1, r2;
-        if (h->prec == SES_C128) {
-            const auto* p = reinterpret_cast<const PlanEntry<double>*>(pp.cp);
-            r0 = p->r0; r1 = p->r1; r2 = p->r2;
-        } else {
-            const auto* p = reinterpret_cast<const PlanEntry<float>*>(pp.cp);
-            r0 = p->r0; r1 = p->r1; r2 = p->r2;
-        }
-        const std::vector<double> t = stage_twiddles(h->n[a], r0, r1, r2);
-        const size_t cnt = t.size() / 2;
-        if (h->prec == SES_C128) {
-            SES_TRY(dalloc(h, &h->stw[a], cnt * sizeof(cx<double>)));
-            SES_CU(cudaMemcpyAsync(h->stw[a], t.data(), cnt * sizeof(cx<double>), cudaMemcpyHostToDevice, h->stream));
-        } else {
-            std::vector<float> hi(2 * cnt), lo(2 * cnt);
-            for (size_t i = 0; i < 2 * cnt; ++i) {
-                hi[i] = (float)t[i];
-                lo[i] = (float)(t[i] - (double)hi[i]);
+        if (pp.cp) {
+            int r0, r1, r2;
+            if (h->prec == SES_C128) {
+                const auto* p = reinterpret_cast<const PlanEntry<double>*>(pp.cp);
+                r0 = p->r0; r1 = p->r1; r2 = p->r2;
+            } else {
+                const auto* p = reinterpret_cast<const PlanEntry<float>*>(pp.cp);
+                r0 = p->r0; r1 = p->r1; r2 = p->r2;
             }
-            SES_TRY(dalloc(h, &h->stw[a], cnt * sizeof(cx<float>)));
-            SES_TRY(dalloc(h, &h->stwl[a], cnt * sizeof(cx<float>)));
-            SES_CU(cudaMemcpyAsync(h->stw[a], hi.data(), cnt * sizeof(cx<float>), cudaMemcpyHostToDevice, h->stream));
-            SES_CU(cudaMemcpyAsync(h->stwl[a], lo.data(), cnt * sizeof(cx<float>), cudaMemcpyHostToDevice, h->stream));
+            SES_TRY(make_twiddles(h, h->n[a], compiled_radices(r0, r1, r2), &h->stw[a], &h->stwl[a]));
+        }
+        if (!pp.cp || (a == 0 && !h->long1d)) {
+            const std::vector<int> rad(pp.g.rad[0], pp.g.rad[0] + pp.g.nst);
+            SES_TRY(make_twiddles(h, h->n[a], rad, &h->ltw[a], &h->ltwl[a]));
         }
     }
     return SES_OK;
@@ -1673,18 +1659,12 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     if (!(h->hsums = static_cast<double*>(pinned_slab().get())))
         return bail(fail(SES_ENOMEM, "pinned host allocation failed"));
     for (int a = 0; a < 3; ++a) {
-        // wavenumber / kinetic tables follow the physical axis (a long line's x
-        // tables cover the whole line); FFT twiddles follow the layout axis
+        // wavenumber / kinetic tables follow the physical axis (a long line's x tables
+        // cover the whole line)
         const int n = std::max(h->n[a], phys_n(h, a));
-        const int nl = h->n[a];
-        if ((st = dalloc(h, &h->tw[a], (size_t)nl * h->esize)) != SES_OK) return bail(st);
         if ((st = dalloc(h, (void**)&h->kv[a], (size_t)n * sizeof(double))) != SES_OK) return bail(st);
         if ((st = dalloc(h, (void**)&h->kd[a], (size_t)n * sizeof(cx<double>))) != SES_OK) return bail(st);
         const unsigned gb = (unsigned)((n + 255) / 256);
-        if (prec == SES_C128)
-            build_twiddles<double><<<gb, 256, 0, h->stream>>>(nl, reinterpret_cast<cx<double>*>(h->tw[a]));
-        else
-            build_twiddles<float><<<gb, 256, 0, h->stream>>>(nl, reinterpret_cast<cx<float>*>(h->tw[a]));
         build_axis_tables<<<gb, 256, 0, h->stream>>>(h->box[2 * a], h->box[2 * a + 1], n,
                                                      with_tables ? dt : 0.0,
                                                      with_tables ? mass : 1.0, h->kv[a], h->kd[a]);
@@ -1707,7 +1687,7 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
                                                                 (cx<float>*)h->tw4l);
     }
     if (cudaGetLastError() != cudaSuccess) return bail(fail(SES_EDEVICE, "axis table build failed"));
-    if ((st = upload_stage_twiddles(h)) != SES_OK) return bail(st);
+    if ((st = make_stage_twiddles(h)) != SES_OK) return bail(st);
     if ((st = dalloc(h, (void**)&h->derr, sizeof(unsigned))) != SES_OK) return bail(st);
     if (!(h->herr = static_cast<unsigned*>(pinned_slab().get())))
         return bail(fail(SES_ENOMEM, "pinned host allocation failed"));

@@ -19,8 +19,6 @@
 
 namespace sesk {
 
-constexpr int kEPTDev = 8;  // elements a thread holds per in-place Stockham stage
-
 enum DiagKind : int { DG_NONE = 0, DG_HALF = 1, DG_FULL = 2 };
 
 // Number of FP64 sums a k-space reduction produces:
@@ -46,10 +44,9 @@ struct Tables {
     const void* tw4;           // W_N^{n1 k2} per element (cx<T>; complex64: FP32-rounded)
     const void* tw4l;          // complex64: FP32 remainder of tw4
     int long_n2;               // N2: stored element (k1, k2) is frequency k2 + N2 k1
-    // dipole drive (drive.ixx:25-40): psi *= cis(-kick u), u = axis . r at cell (i, j, k),
-    // r = origin + index * spacing; kick = 0 off
-    double kick;
-    double kax[3], korg[3], kh[3];
+    // dipole drive (drive.ixx:25-40): the per-axis factors of this pass's kick
+    // psi *= cis(-theta (axis . r)), nx + ny + nz entries; null off
+    const cx<double>* kick;
 };
 
 // complex64 phase multiplies in FP32 on the delta form: psi + psi*d, d = factor - 1.
@@ -66,7 +63,7 @@ template <typename T>
 struct PassArgs {
     const cx<T>* src;
     cx<T>* dst;
-    Geo g;
+    LinePlan g;
     int axis;  // 0 = x (contiguous lines), 1 = y, 2 = z
     int nx, ny, nz;
     long long nlines;
@@ -74,8 +71,7 @@ struct PassArgs {
     // element stride se.  For the x axis: base = s * nx, se = 1.
     long long nu, sw, se;
     FastDiv fnu, fny, fnx;
-    const cx<T>* tw;   // twiddles cis(-2 pi t / n), t < n (run-time plans)
-    const cx<T>* stw;  // per-stage twiddle tables of a compiled plan (hi part)
+    const cx<T>* stw;  // per-stage twiddle tables of the axis's plan, forward then reversed order (hi part)
     const cx<T>* stwl; // FP32: remainder (lo part) of the same tables
     // run-time parts of the pass program (the structure is the kernel's MODE)
     int d_load, d_mid, d_store;
@@ -95,48 +91,12 @@ __device__ __forceinline__ double maskval(const Tables& tb, long long f, int i, 
 template <typename T>
 __device__ __forceinline__ cx<T> apply_diag_tv(cx<T> v, int kind, cx<T> tab, int use_mask, double m);
 
-// Dipole kick of cell (i, j, k): psi * cis(-kick (ax x + ay y + az z)), the phase in FP64;
-// complex64 multiplies in FP32 on the delta form.  Out of line: the FP64 sincos
-// stays out of the passes' register allocation, which only test kick != 0.
-template <typename T>
-__device__ __noinline__ cx<T> kick_apply(cx<T> v, double kick, double ax, double ay, double az, double x0,
-                                         double y0, double z0, double hx, double hy, double hz, int i, int j,
-                                         int k) {
-    const double u = ax * (x0 + i * hx) + ay * (y0 + j * hy) + az * (z0 + k * hz);
-    const double ang = -kick * u;
-    if constexpr (sizeof(T) == 4) {
-        double s2, c2;
-        sincos(0.5 * ang, &s2, &c2);
-        return add_mul(v, mk<float>((float)(-2.0 * s2 * s2), (float)(2.0 * s2 * c2)));
-    } else {
-        double s, c;
-        sincos(ang, &s, &c);
-        return v * mk<double>(c, s);
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ cx<T> kick_mul(cx<T> v, const Tables& tb, int i, int j, int k) {
-    if (tb.kick == 0.0) return v;
-    return kick_apply<T>(v, tb.kick, tb.kax[0], tb.kax[1], tb.kax[2], tb.korg[0], tb.korg[1], tb.korg[2], tb.kh[0],
-                         tb.kh[1], tb.kh[2], i, j, k);
-}
-
 // psi * (potential phase) * (mask) at flat index f, coordinates (i, j, k).
 template <typename T>
 __device__ __forceinline__ cx<T> apply_diag(cx<T> v, int kind, int use_mask, long long f, int i, int j,
                                             int k, const Tables& tb) {
     const cx<T> tab = kind != DG_NONE ? reinterpret_cast<const cx<T>*>(tb.vtab)[f] : v;
     return apply_diag_tv(v, kind, tab, use_mask, use_mask ? maskval<T>(tb, f, i, j, k) : 1.0);
-}
-
-// The same and the dipole kick: only the run-time-plan x pass carries the kick,
-// which keeps its FP64 phase code out of the compiled passes' register budget
-// (driven steps always run their x passes on those kernels).
-template <typename T>
-__device__ __forceinline__ cx<T> apply_diag_kick(cx<T> v, int kind, int use_mask, long long f, int i, int j,
-                                                 int k, const Tables& tb) {
-    return kick_mul(apply_diag(v, kind, use_mask, f, i, j, k, tb), tb, i, j, k);
 }
 
 // Same as apply_diag with the potential-table entry and mask value supplied
@@ -288,223 +248,11 @@ enum SModeK : int {
 };
 constexpr int kSModes = 7;
 
-// ---------------------------------------------------------------------------
-// Contiguous-axis (x) pass.  Tile = L consecutive x-lines, loaded and stored
-// with coalesced accesses; shared layout [l][e] with an odd pitch.
-// ---------------------------------------------------------------------------
 // Programmatic dependent launch: a pass kernel may be launched while the
 // previous kernel of its stream drains; it waits here, before touching any
 // field or argument table, until that kernel has completed and its writes are
 // visible (a no-op for a normal launch).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename T, int MODE>
-__global__ void __launch_bounds__(512, 1) xpass_kernel(const PassArgs<T> a) {
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ Geo g;  // stage tables are indexed at run time: keep them out of parameter space
-    if (threadIdx.x == 0) g = a.g;
-    cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-    const int n = a.g.n, L = a.g.L;
-    const long long m0 = (long long)blockIdx.x * L;
-    const int tile = L * n;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    constexpr bool kDiagLoad = MODE == XM_START || MODE == XM_1D;
-    constexpr bool kDiagStore = MODE == XM_END || MODE == XM_1D;
-
-    // load (coalesced), optional real-space diagonal
-    for (int idx = tid; idx < tile; idx += nt) {
-        const int l = (int)fdiv((uint32_t)idx, a.g.fn), e = idx - l * n;
-        const long long m = m0 + l;
-        cx<T> v = mk<T>((T)0, (T)0);
-        if (m < a.nlines) {
-            const long long f = m * n + e;
-            v = a.src[f];
-            if constexpr (kDiagLoad) {
-                if (a.d_load != DG_NONE || a.m_load) {
-                    const int k = (int)fdiv((uint32_t)m, a.fny);
-                    const int j = (int)(m - (long long)k * a.ny);
-                    v = apply_diag_kick(v, a.d_load, a.m_load, f, e, j, k, a.tb);
-                }
-            }
-        }
-        sm[l * a.g.ls + e] = v;
-    }
-    __syncthreads();
-
-    auto lds = [&](int l, int e) -> cx<T> { return sm[l * g.ls + e]; };
-    auto sts = [&](int l, int e, cx<T> v) { sm[l * g.ls + e] = v; };
-
-    if constexpr (MODE == XM_INV || MODE == XM_MID || MODE == XM_END) {
-        auto ldc = [&](int l, int e) -> cx<T> { return cconj(sm[l * g.ls + e]); };
-        auto stc = [&](int l, int e, cx<T> v) {
-            sm[l * g.ls + e] = MODE == XM_INV ? scale_d(cconj(v), a.out_scale) : cconj(v);
-        };
-        fft_tile<T, kEPTDev, false, false>(g, sm, a.tw, ldc, stc);
-    }
-    if constexpr (MODE == XM_MID) {
-        if (a.d_mid != DG_NONE || a.m_mid) {
-            for (int idx = tid; idx < tile; idx += nt) {
-                const int l = (int)fdiv((uint32_t)idx, g.fn), e = idx - l * n;
-                const long long m = m0 + l;
-                if (m < a.nlines) {
-                    const int k = (int)fdiv((uint32_t)m, a.fny);
-                    const int j = (int)(m - (long long)k * a.ny);
-                    sm[l * g.ls + e] =
-                        apply_diag_kick(sm[l * g.ls + e], a.d_mid, a.m_mid, m * n + e, e, j, k, a.tb);
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if constexpr (MODE == XM_FWD || MODE == XM_START || MODE == XM_MID) {
-        fft_tile<T, kEPTDev, false, false>(g, sm, a.tw, lds, sts);
-    }
-    if constexpr (MODE == XM_1D) {
-        // x is the only transformed axis: fwd, K/N, inverse, all in the tile
-        auto stk = [&](int l, int e, cx<T> v) {
-            const long long m0l = m0 + l;
-            const long long m = m0l < a.nlines ? m0l : 0;
-            const int k = (int)fdiv((uint32_t)m, a.fny);
-            const int j = (int)(m - (long long)k * a.ny);
-            sm[l * g.ls + e] = kinetic_apply(v, dmul1(a.tb.kd[1][j], a.tb.kd[2][k]), a.tb.kd[0], a.tb.kdf[0],
-                                             e, a.tb.kscale);
-        };
-        fft_tile<T, kEPTDev, false, false>(g, sm, a.tw, lds, stk);
-        auto stc = [&](int l, int e, cx<T> v) { sm[l * g.ls + e] = cconj(v); };
-        fft_tile<T, kEPTDev, false, false>(g, sm, a.tw, lds, stc);
-    }
-    if constexpr (MODE == XM_REDUCE) {
-        double acc[kRedK] = {0, 0, 0, 0, 0};
-        auto str = [&](int l, int e, cx<T> v) {
-            const long long m = m0 + l;
-            if (m < a.nlines) {
-                const int k = (int)fdiv((uint32_t)m, a.fny);
-                const int j = (int)(m - (long long)k * a.ny);
-                const double k3[3] = {a.tb.kv[0][e], a.tb.kv[1][j], a.tb.kv[2][k]};
-                const cx<double> p = widen(v);
-                acc_k(acc, p.x * p.x + p.y * p.y, k3, a.tb.inv_mass);
-            }
-        };
-        fft_tile<T, kEPTDev, false, false>(g, sm, a.tw, lds, str);
-        block_reduce_store<kRedK>(acc, a.partials);
-        return;
-    }
-
-    // store (coalesced), optional real-space diagonal
-    if constexpr (MODE != XM_REDUCE) for (int idx = tid; idx < tile; idx += nt) {
-        const int l = (int)fdiv((uint32_t)idx, g.fn), e = idx - l * n;
-        const long long m = m0 + l;
-        if (m < a.nlines) {
-            const long long f = m * n + e;
-            cx<T> v = sm[l * g.ls + e];
-            if constexpr (kDiagStore) {
-                if (a.d_store != DG_NONE || a.m_store) {
-                    const int k = (int)fdiv((uint32_t)m, a.fny);
-                    const int j = (int)(m - (long long)k * a.ny);
-                    v = apply_diag_kick(v, a.d_store, a.m_store, f, e, j, k, a.tb);
-                }
-            }
-            a.dst[f] = v;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Strided-axis (y or z) pass.  Tile = L line slots whose first elements are
-// consecutive in memory, so every element load/store of a warp is a
-// contiguous run.  Stage 0 reads HBM directly and the last stage writes HBM
-// directly; intermediate stages use the shared tile ([e][l] layout).
-// ---------------------------------------------------------------------------
-template <typename T, int MODE>
-__global__ void __launch_bounds__(512, 1) spass_kernel(const PassArgs<T> a) {
-    pdl_wait();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ Geo g;  // stage tables are indexed at run time: keep them out of parameter space
-    if (threadIdx.x == 0) g = a.g;
-    const int n = a.g.n, L = a.g.L;
-    cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-    // per-line data after the tile, 16-byte aligned: kinetic delta of the two
-    // other axes, their wavenumbers, and the line's base offset in psi
-    cx<double>* dother =
-        reinterpret_cast<cx<double>*>(smraw + (((size_t)L * n * sizeof(cx<T>) + 15) & ~(size_t)15));
-    double* kq = reinterpret_cast<double*>(dother + L);
-    long long* lbase = reinterpret_cast<long long*>(kq + 2 * L);
-    const long long s0 = (long long)blockIdx.x * L;
-    constexpr bool kLineInfo = MODE == SM_FUSED || MODE == SM_REDUCE;
-    // the two other axes, in increasing order: y-pass -> (x, z), z-pass -> (x, y)
-    const bool ypass = a.axis == 1;
-    const cx<double>* kd1 = a.tb.kd[0];
-    const cx<double>* kd2 = ypass ? a.tb.kd[2] : a.tb.kd[1];
-    const cx<double>* kda = ypass ? a.tb.kd[1] : a.tb.kd[2];
-    const double* kv1 = a.tb.kv[0];
-    const double* kv2 = ypass ? a.tb.kv[2] : a.tb.kv[1];
-    const double* kva = ypass ? a.tb.kv[1] : a.tb.kv[2];
-
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-        const long long s = s0 + l;
-        long long base = -1;
-        int c1 = 0, c2 = 0;
-        if (s < a.nlines) {
-            const long long w = (long long)fdiv((uint32_t)s, a.fnu);
-            const long long u = s - w * a.nu;
-            base = u + w * a.sw;
-            if (ypass) {  // lines (i, k)
-                c1 = (int)u;
-                c2 = (int)w;
-            } else {  // z: lines (i, j), u = i + nx j
-                c2 = (int)fdiv((uint32_t)u, a.fnx);
-                c1 = (int)(u - (long long)c2 * a.nx);
-            }
-        }
-        lbase[l] = base;
-        if constexpr (kLineInfo) {
-            dother[l] = dmul1(kd1[c1], kd2[c2]);
-            kq[2 * l] = kv1[c1];
-            kq[2 * l + 1] = kv2[c2];
-        }
-    }
-    __syncthreads();
-
-    const long long se = a.se;
-    auto ldg = [&](int l, int e) -> cx<T> {
-        const long long b = lbase[l];
-        return b >= 0 ? a.src[b + e * se] : mk<T>((T)0, (T)0);
-    };
-    auto stg = [&](int l, int e, cx<T> v) {
-        const long long b = lbase[l];
-        if (b >= 0) a.dst[b + e * se] = v;
-    };
-
-    if constexpr (MODE == SM_FWD) {
-        fft_tile<T, kEPTDev, true, true>(g, sm, a.tw, ldg, stg);
-    } else if constexpr (MODE == SM_INV) {
-        auto ldc = [&](int l, int e) -> cx<T> { return cconj(ldg(l, e)); };
-        auto stc = [&](int l, int e, cx<T> v) { stg(l, e, scale_d(cconj(v), a.out_scale)); };
-        fft_tile<T, kEPTDev, true, true>(g, sm, a.tw, ldc, stc);
-    } else if constexpr (MODE == SM_FUSED) {
-        auto stk = [&](int l, int e, cx<T> v) {
-            sm[l * g.ls + e * g.es] = kinetic_apply(v, dother[l], kda, ypass ? a.tb.kdf[1] : a.tb.kdf[2], e,
-                                                    a.tb.kscale);
-        };
-        fft_tile<T, kEPTDev, true, false>(g, sm, a.tw, ldg, stk);
-        auto lds = [&](int l, int e) -> cx<T> { return sm[l * g.ls + e * g.es]; };
-        auto stc = [&](int l, int e, cx<T> v) { stg(l, e, cconj(v)); };
-        fft_tile<T, kEPTDev, false, true>(g, sm, a.tw, lds, stc);
-    } else {  // SM_REDUCE
-        double acc[kRedK] = {0, 0, 0, 0, 0};
-        auto str = [&](int l, int e, cx<T> v) {
-            if (lbase[l] >= 0) {
-                const double ka = kva[e], kb = kq[2 * l + 1];
-                const double k3[3] = {kq[2 * l], ypass ? ka : kb, ypass ? kb : ka};
-                const cx<double> p = widen(v);
-                acc_k(acc, p.x * p.x + p.y * p.y, k3, a.tb.inv_mass);
-            }
-        };
-        fft_tile<T, kEPTDev, true, true>(g, sm, a.tw, ldg, str);
-        block_reduce_store<kRedK>(acc, a.partials);
-    }
-}
 
 // The grid as the real-space observables see it.
 struct ObsArgs {
