@@ -276,8 +276,7 @@ struct ses_solver {
     static constexpr int kMaxVar = 4;
     CUtensorMap tmap[2][3][kMaxVar];
     bool tmap_ok[2][3][kMaxVar] = {};
-    unsigned* derr = nullptr;  // device error word written by bounded waits
-    unsigned* herr = nullptr;  // pinned host copy
+    unsigned* herr = nullptr;  // error word (page-locked) that the device's bounded waits set
     int sms = 148;
     bool pipelined = true;
     bool pdl = true;  // single-field passes launched with programmatic stream serialization
@@ -376,7 +375,7 @@ void release(ses_solver* h) {
         if (p) cudaFreeAsync(p, fs);
     };
     void* ptrs[] = {h->psi, h->scratch, h->vtab, h->V, h->maskfull, h->partials, h->kpartials, h->dsums, h->kfull, h->tw4, h->tw4l,
-                    h->dobs, h->derr, h->kicks};
+                    h->dobs, h->kicks};
     for (void* p : ptrs) dfree(p);
     for (int a = 0; a < 3; ++a) {
         dfree(h->kv[a]);
@@ -402,31 +401,36 @@ void set_smem_attr(K kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 }
 
-// Bounded wait on everything queued so far on the handle's stream.
-ses_status wait_bounded(ses_solver* h, int timeout_ms) {
-    if (timeout_ms <= 0) timeout_ms = 10000;
-    if (h->derr) SES_CU(cudaMemcpyAsync(h->herr, h->derr, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
-    SES_CU(cudaEventRecord(h->ev, h->stream));
+// Polls an event until it completes (cudaSuccess), fails, or timeout_ms has passed
+// (cudaErrorNotReady).  Readings are a few us to a few ms away: the first 2 ms poll
+// back to back, since a sleep of 20 us takes about 75 (the kernel's timer slack), after
+// that between sleeps.
+cudaError_t poll_event(cudaEvent_t e, int timeout_ms) {
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
-        const cudaError_t q = cudaEventQuery(h->ev);
-        if (q == cudaSuccess) {
-            if (h->herr && *h->herr) {
-                *h->herr = 0;
-                cudaMemsetAsync(h->derr, 0, sizeof(unsigned), h->stream);
-                return fail(SES_ETIMEDOUT, "a pipelined pass gave up waiting for its tile loads");
-            }
-            return SES_OK;
-        }
-        if (q != cudaErrorNotReady)
-            return fail(SES_EDEVICE, std::string("device error: ") + cudaGetErrorString(q));
-        const auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(
-                            std::chrono::steady_clock::now() - t0)
-                            .count();
-        if (ms > timeout_ms)
-            return fail(SES_ETIMEDOUT, "wait exceeded " + std::to_string(timeout_ms) + " ms");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+        const cudaError_t q = cudaEventQuery(e);
+        if (q != cudaErrorNotReady) return q;
+        const auto waited = std::chrono::steady_clock::now() - t0;
+        if (waited > std::chrono::milliseconds(timeout_ms)) return q;
+        if (waited > std::chrono::milliseconds(2)) std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
+}
+
+// Bounded wait on everything queued so far on the handle's stream.  A pass whose own
+// bounded wait ran out has set the error word, which is page-locked host memory.
+ses_status wait_bounded(ses_solver* h, int timeout_ms) {
+    if (timeout_ms <= 0) timeout_ms = 10000;
+    SES_CU(cudaEventRecord(h->ev, h->stream));
+    switch (poll_event(h->ev, timeout_ms)) {
+        case cudaSuccess: break;
+        case cudaErrorNotReady: return fail(SES_ETIMEDOUT, "wait exceeded " + std::to_string(timeout_ms) + " ms");
+        default: return fail(SES_EDEVICE, std::string("device error: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    if (h->herr && *h->herr) {
+        *h->herr = 0;
+        return fail(SES_ETIMEDOUT, "a pipelined pass gave up waiting for its tile loads");
+    }
+    return SES_OK;
 }
 
 template <typename T>
@@ -533,7 +537,7 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
             const auto& v = e->xv[xs];
             PipeArgs pa{};
             pa.ntiles = (int)((pp.nlines + v.lpc - 1) / v.lpc);
-            pa.err = h->derr;
+            pa.err = h->herr;
             pa.wait_limit = h->wait_limit;
             pa.extra_tx = h->extra_tx;
             const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
@@ -551,7 +555,7 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
                 pa.kind = axis == 1 ? 0 : 1;
                 pa.rows_per_box = n > 256 ? 256 : n;
                 pa.nbox = n / pa.rows_per_box;
-                pa.err = h->derr;
+                pa.err = h->herr;
                 pa.wait_limit = h->wait_limit;
                 pa.extra_tx = h->extra_tx;
                 const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
@@ -1688,12 +1692,9 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     }
     if (cudaGetLastError() != cudaSuccess) return bail(fail(SES_EDEVICE, "axis table build failed"));
     if ((st = make_stage_twiddles(h)) != SES_OK) return bail(st);
-    if ((st = dalloc(h, (void**)&h->derr, sizeof(unsigned))) != SES_OK) return bail(st);
     if (!(h->herr = static_cast<unsigned*>(pinned_slab().get())))
         return bail(fail(SES_ENOMEM, "pinned host allocation failed"));
     *h->herr = 0;
-    if (cudaMemsetAsync(h->derr, 0, sizeof(unsigned), h->stream) != cudaSuccess)
-        return bail(fail(SES_EDEVICE, "memset failed"));
     cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->dev);
     if (const char* env = std::getenv("SES_PIPELINED")) h->pipelined = std::atoi(env) != 0;
     build_tmaps(h, 0, h->psi);
@@ -1853,8 +1854,7 @@ struct ses_batch_s {
     int dev = 0;
     cudaStream_t own = nullptr, stream = nullptr;
     cudaEvent_t fork = nullptr, ev = nullptr;
-    unsigned* derr = nullptr;  // device error word of the pipelined batched passes
-    unsigned* herr = nullptr;  // pinned host copy
+    unsigned* herr = nullptr;  // error word (page-locked) of the pipelined batched passes
     std::vector<ses_solver*> members;  // in add order
     std::vector<BatchClass*> classes;
     std::map<std::string, int> sel;    // autotuned variant per class pass (batch_tune_key)
@@ -1867,16 +1867,7 @@ struct ses_batch_s {
 namespace {
 
 // Host wait (polling, bounded) for an event; false on timeout or device error.
-bool event_wait(cudaEvent_t e, int timeout_ms) {
-    const auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        const cudaError_t q = cudaEventQuery(e);
-        if (q == cudaSuccess) return true;
-        if (q != cudaErrorNotReady) return false;
-        if (std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(timeout_ms)) return false;
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
-    }
-}
+bool event_wait(cudaEvent_t e, int timeout_ms) { return poll_event(e, timeout_ms) == cudaSuccess; }
 
 // A class graph that queued launches may still use: destroyed later (reap).
 void retire_graph(ses_batch_s* b, cudaGraphExec_t g) {
@@ -1930,28 +1921,18 @@ void drop_class(ses_batch_s* b, BatchClass* c) {
 
 ses_status batch_wait(ses_batch_s* b, int timeout_ms) {
     if (timeout_ms <= 0) timeout_ms = 10000;
-    SES_CU(cudaMemcpyAsync(b->herr, b->derr, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
     SES_CU(cudaEventRecord(b->ev, b->stream));
-    const auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        const cudaError_t q = cudaEventQuery(b->ev);
-        if (q == cudaSuccess) {
-            reap(b, false);
-            if (*b->herr) {
-                *b->herr = 0;
-                cudaMemsetAsync(b->derr, 0, sizeof(unsigned), b->stream);
-                return fail(SES_ETIMEDOUT, "a pipelined batched pass gave up waiting for its tile loads");
-            }
-            return SES_OK;
-        }
-        if (q != cudaErrorNotReady)
-            return fail(SES_EDEVICE, std::string("device error: ") + cudaGetErrorString(q));
-        const auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(
-                            std::chrono::steady_clock::now() - t0)
-                            .count();
-        if (ms > timeout_ms) return fail(SES_ETIMEDOUT, "wait exceeded " + std::to_string(timeout_ms) + " ms");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+    switch (poll_event(b->ev, timeout_ms)) {
+        case cudaSuccess: break;
+        case cudaErrorNotReady: return fail(SES_ETIMEDOUT, "wait exceeded " + std::to_string(timeout_ms) + " ms");
+        default: return fail(SES_EDEVICE, std::string("device error: ") + cudaGetErrorString(cudaGetLastError()));
     }
+    reap(b, false);
+    if (*b->herr) {
+        *b->herr = 0;
+        return fail(SES_ETIMEDOUT, "a pipelined batched pass gave up waiting for its tile loads");
+    }
+    return SES_OK;
 }
 
 template <typename T>
@@ -2277,7 +2258,7 @@ ses_status class_launch(const ses_batch_s* b, const BatchClass& c, int prog, boo
                                        : c.svar[q] >= 0)) {
         const int n = h0->n[axis];
         PipeArgs pa{};
-        pa.err = b->derr;
+        pa.err = b->herr;
         BatchWork w{};
         if (axis == 0) {
             const auto& v = e->xv[c.xvar];
@@ -3070,11 +3051,8 @@ ses_status ses_batch_create(ses_batch* out) {
         delete b;
         return fail(SES_EDEVICE, "batch stream creation failed (no device?)");
     }
-    if (cudaMalloc(&b->derr, sizeof(unsigned)) != cudaSuccess ||
-        cudaMallocHost(&b->herr, sizeof(unsigned)) != cudaSuccess ||
-        cudaMemset(b->derr, 0, sizeof(unsigned)) != cudaSuccess) {
+    if (cudaMallocHost(&b->herr, sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
-        if (b->derr) cudaFree(b->derr);
         cudaEventDestroy(b->ev);
         cudaEventDestroy(b->fork);
         cudaStreamDestroy(b->own);
@@ -3097,7 +3075,6 @@ ses_status ses_batch_destroy(ses_batch b) {
     for (BatchClass* c : b->classes) drop_class(b, c);
     cudaStreamSynchronize(b->stream);
     reap(b, true);
-    if (b->derr) cudaFree(b->derr);
     if (b->herr) cudaFreeHost(b->herr);
     if (b->ev) cudaEventDestroy(b->ev);
     if (b->fork) cudaEventDestroy(b->fork);
