@@ -197,6 +197,47 @@ __global__ void build_axis_tables_imag(int n, double dtau, double mass, const do
     if (j < n) kd[j] = mk<double>(expm1(theta_k(__dmul_rn(kv[j], kv[j]), mass, dtau)), 0.0);
 }
 
+// Smallest and largest potential value, for the range that one imaginary-time step can
+// scale a field by: one row per CTA, then (one CTA) host[0] = min, host[1] = max.
+__global__ void __launch_bounds__(256) value_range(const double* __restrict__ V, long long N, double* rows) {
+    double lo = INFINITY, hi = -INFINITY;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < N; i += (long long)gridDim.x * 256) {
+        lo = fmin(lo, V[i]);
+        hi = fmax(hi, V[i]);
+    }
+    __shared__ double slo[256], shi[256];
+    slo[threadIdx.x] = lo;
+    shi[threadIdx.x] = hi;
+    __syncthreads();
+    for (int h = 128; h > 0; h >>= 1) {
+        if ((int)threadIdx.x < h) {
+            slo[threadIdx.x] = fmin(slo[threadIdx.x], slo[threadIdx.x + h]);
+            shi[threadIdx.x] = fmax(shi[threadIdx.x], shi[threadIdx.x + h]);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        rows[2 * blockIdx.x] = slo[0];
+        rows[2 * blockIdx.x + 1] = shi[0];
+    }
+}
+
+__global__ void value_range_fold(const double* __restrict__ rows, int n, double* host) {
+    double lo = INFINITY, hi = -INFINITY;
+    for (int i = threadIdx.x; i < n; i += 32) {
+        lo = fmin(lo, rows[2 * i]);
+        hi = fmax(hi, rows[2 * i + 1]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_down_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_down_sync(0xffffffffu, hi, o));
+    }
+    if (threadIdx.x == 0) {
+        host[0] = lo;
+        host[1] = hi;
+    }
+}
+
 // psi *= 1 / sqrt(sum |psi|^2 dV), the sum taken from sums[0] on the device;
 // sums[0] is kept for the energy estimate.
 template <typename T>

@@ -294,6 +294,7 @@ struct ses_solver {
     // transformed in four steps; box[0..1] and N keep the physical line
     bool long1d = false;
     bool imag = false;       // imaginary-time handle: real weight tables, no absorber
+    double vmin = 0.0, vmax = 0.0;  // of an imaginary-time handle's potential
     void* kfull = nullptr;   // kinetic delta per stored k-space element
     void* tw4 = nullptr;     // W_N^{n1 k2} per element (complex64: hi part)
     void* tw4l = nullptr;    // complex64: lo part
@@ -907,19 +908,40 @@ ses_status enqueue_fft3(ses_solver* h, void* data, int inverse) {
 
 ObsArgs obs_args(const ses_solver* h, double xlo, double xhi);
 
-// Imaginary time: psi /= sqrt(sum |psi|^2 dV) on the device (the sum stays in dsums[0]).
+// Imaginary time: psi /= sqrt(sum |psi|^2 dV) on the device (the sum stays in dsums[0]
+// and, page-locked, in hsums[0]).
 template <typename T>
 ses_status enqueue_renormalize(ses_solver* h) {
     cudaStream_t s = h->stream;
-    const ObsArgs o = obs_args(h, -1e300, 1e300);
-    const unsigned ob = obs_blocks(h->N, kObsBlocks);
-    obs_real_kernel<T><<<ob, 256, 0, s>>>(reinterpret_cast<const cx<T>*>(h->psi), h->V, o, h->partials);
-    finalize_kernel<<<1, kFoldThreads, 0, s>>>(h->partials, (int)ob, nullptr, 0, h->dsums, nullptr);
-    const double dv = o.hx * o.hy * o.hz;
+    cx<T>* psi = reinterpret_cast<cx<T>*>(h->psi);
+    const ObsArgs o = obs_args(h, 0.0, 0.0);
+    norm_peak_kernel<T><<<kNormPeakBlocks, 256, 0, s>>>(psi, h->N, h->partials);
+    norm_peak_finalize<<<1, 256, 0, s>>>(h->partials, kNormPeakBlocks, h->dsums, h->hsums);
     const unsigned gb = (unsigned)std::min<long long>((h->N + 255) / 256, 148 * 16);
-    renormalize_kernel<T><<<gb, 256, 0, s>>>(reinterpret_cast<cx<T>*>(h->psi), h->N, h->dsums, dv);
+    renormalize_kernel<T><<<gb, 256, 0, s>>>(psi, h->N, h->dsums, o.hx * o.hy * o.hz);
     SES_CU(cudaGetLastError());
     return SES_OK;
+}
+
+// Steps of a normalised field that imaginary time may run before its scale could leave
+// the storage type's range.  A step is linear and multiplies the field's norm by
+// something between exp(-(max(V, 0) + k^2/(2m)) dtau) and exp(-min(V, 0) dtau), so a
+// renormalisation between two steps changes nothing but rounding, and steps within
+// the range run merged like those of real time (one kick instead of two, no batch end
+// and start, no norm in between).  Kept: a factor e^48 either way in complex64 (type
+// range e^+-87, transform sums up to N), e^250 in complex128 (the norm is of squares,
+// range e^+-708); at most 33 steps, 4 captured graphs.  64^3 complex128,
+// renormalised after every step: 35 -> 14 us a step.
+int relax_run(const ses_solver* h) {
+    double kmax = 0.0;
+    for (int a = 0; a < 3; ++a)
+        if (phys_n(h, a) > 1) {
+            const double k = 3.14159265358979323846 * phys_n(h, a) / (h->box[2 * a + 1] - h->box[2 * a]);
+            kmax += 0.5 * k * k / h->mass;
+        }
+    const double per_step = h->dt * std::max(std::max(h->vmax, 0.0) + kmax, std::max(-h->vmin, 0.0));
+    const double most = (h->prec == SES_C128 ? 250.0 : 48.0) / per_step;
+    return most >= 33.0 ? 33 : (most >= 2.0 ? (int)most : 1);  // also 1 when V is not finite
 }
 
 ObsArgs obs_args(const ses_solver* h, double xlo, double xhi) {
@@ -1402,6 +1424,9 @@ ses_status build_tables(ses_solver* h) {
             build_vtab_imag_c128<<<gb, tb, 0, h->stream>>>(h->V, reinterpret_cast<cx<double>*>(h->vtab), N, h->dt);
         else
             build_vtab_imag_c64<<<gb, tb, 0, h->stream>>>(h->V, reinterpret_cast<cx<float>*>(h->vtab), N, h->dt);
+        // h->vmin, vmax, read once the stream has passed (read_value_range)
+        value_range<<<kObsBlocks, 256, 0, h->stream>>>(h->V, N, h->partials);
+        value_range_fold<<<1, 32, 0, h->stream>>>(h->partials, kObsBlocks, h->hsums + 16);
         SES_CU(cudaGetLastError());
         return SES_OK;
     }
@@ -1413,6 +1438,13 @@ ses_status build_tables(ses_solver* h) {
                                                   h->dt);
     SES_CU(cudaGetLastError());
     return SES_OK;
+}
+
+// The range build_tables found, after a wait on the stream.
+void read_value_range(ses_solver* h) {
+    if (!h->imag) return;
+    h->vmin = h->hsums[16];
+    h->vmax = h->hsums[17];
 }
 
 void attach_compiled_plan(ses_solver* h, int axis) {
@@ -1716,6 +1748,7 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
             return bail(fail(SES_EDEVICE, "memset failed"));
     }
     if ((st = wait_bounded(h, 0)) != SES_OK) return bail(st);
+    read_value_range(h);
     *out = h;
     return SES_OK;
 }
@@ -2631,15 +2664,23 @@ ses_status ses_gpu_relax(ses_handle h, int nsteps, int renorm_every, double* ene
     if (!h->imag) return fail(SES_EINVAL, "handle was not created for imaginary time (ses_gpu_create_imag)");
     if (nsteps < 1) return fail(SES_EINVAL, "nsteps must be >= 1");
     const int R = renorm_every > 0 ? renorm_every : 1;
-    int done = 0, last = 1;
-    while (done < nsteps) {
-        last = std::min(R, nsteps - done);
-        SES_TRY(h->prec == SES_C128 ? enqueue_steps<double>(h, last, false) : enqueue_steps<float>(h, last, false));
-        SES_TRY(h->prec == SES_C128 ? enqueue_renormalize<double>(h) : enqueue_renormalize<float>(h));
-        done += last;
+    const int last = nsteps - (nsteps - 1) / R * R;  // steps of the last renormalisation, the energy's
+    auto run = [&](int steps) -> ses_status {
+        SES_TRY(h->prec == SES_C128 ? enqueue_steps<double>(h, steps, false) : enqueue_steps<float>(h, steps, false));
+        return h->prec == SES_C128 ? enqueue_renormalize<double>(h) : enqueue_renormalize<float>(h);
+    };
+    int left = nsteps - last;
+    if (left > 0) {  // the caller's field has any norm: its first renormalisation comes as asked for
+        SES_TRY(run(R));
+        left -= R;
     }
+    for (const int most = std::max(R, relax_run(h)); left > 0;) {
+        const int steps = std::min(most, left);
+        SES_TRY(run(steps));
+        left -= steps;
+    }
+    SES_TRY(run(last));
     if (!energy) return SES_OK;
-    SES_CU(cudaMemcpyAsync(h->hsums, h->dsums, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     SES_TRY(wait_bounded(h, 0));
     const ObsArgs o = obs_args(h, 0.0, 0.0);
     const double n2 = h->hsums[0] * o.hx * o.hy * o.hz;  // norm^2 after the last `last` steps
@@ -2660,7 +2701,9 @@ ses_status ses_gpu_set_potential(ses_handle h, const double* V) {
     if (!h->with_tables) return fail(SES_EINVAL, "handle has no phase tables");
     SES_CU(cudaMemcpyAsync(h->V, V, h->N * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     SES_TRY(h->prec == SES_C128 ? build_tables<double>(h) : build_tables<float>(h));
-    return wait_bounded(h, 0);
+    SES_TRY(wait_bounded(h, 0));
+    read_value_range(h);
+    return SES_OK;
 }
 
 ses_status ses_gpu_set_absorber_separable(ses_handle h, const double* mx, const double* my,
