@@ -24,6 +24,7 @@
 #include "ses_aux.cuh"
 #include "ses_engine.cuh"
 #include "ses_line.cuh"
+#include "ses_longline.cuh"
 #include "ses_pass.cuh"
 #include "ses_plans.cuh"
 #include "ses_plane.cuh"
@@ -111,6 +112,8 @@ struct Registry {
     std::vector<PlanEntry<double>> d;
     std::vector<PlaneEntry<float>> pf;  // plane passes of the two-sweep step
     std::vector<PlaneEntry<double>> pd;
+    std::vector<LongEntry<float>> lf;   // long lines held by one cluster
+    std::vector<LongEntry<double>> ld;
 };
 
 const Registry& registry() {
@@ -122,6 +125,7 @@ const Registry& registry() {
         register_plans_256(r.f, r.d);
         register_plans_large(r.f, r.d);
         register_planes(r.pf, r.pd);
+        register_long_lines(r.lf, r.ld);
     });
     return r;
 }
@@ -295,6 +299,7 @@ struct ses_solver {
     bool long1d = false;
     bool imag = false;       // imaginary-time handle: real weight tables, no absorber
     double vmin = 0.0, vmax = 0.0;  // of an imaginary-time handle's potential
+    const void* longk = nullptr;  // the cluster kernel of the line's whole steps (nullptr: two launches a step)
     void* kfull = nullptr;   // kinetic delta per stored k-space element
     void* tw4 = nullptr;     // W_N^{n1 k2} per element (complex64: hi part)
     void* tw4l = nullptr;    // complex64: lo part
@@ -692,6 +697,57 @@ void init_kernel_attrs() {  // once per process; handles may be created from sev
     });
 }
 
+// The long-line kernel built for the line's plans, the one on the most CTAs that the
+// device can hold (SES_LONG: 0 none, else the CTAs of the cluster).
+template <typename T>
+const void* find_long(const ses_solver* h) {
+    if (!h->long1d || h->imag) return nullptr;
+    const auto* px = reinterpret_cast<const PlanEntry<T>*>(h->pp[0].cp);
+    const auto* py = reinterpret_cast<const PlanEntry<T>*>(h->pp[1].cp);
+    if (!px || !py) return nullptr;
+    const char* env = std::getenv("SES_LONG");
+    const auto& v = [] () -> const std::vector<LongEntry<T>>& {
+        if constexpr (sizeof(T) == 4) return registry().lf;
+        else return registry().ld;
+    }();
+    for (const auto& e : v)
+        if (e.usable && e.n1 == h->n[0] && e.n2 == h->n[1] && (!env || std::atoi(env) == e.cs) && e.xe == px->e &&
+            e.xr[0] == px->r0 && e.xr[1] == px->r1 && e.xr[2] == px->r2 && e.ye == py->e && e.yr[0] == py->r0 &&
+            e.yr[1] == py->r1 && e.yr[2] == py->r2)
+            return &e;
+    return nullptr;
+}
+
+// S steps of a long line by its cluster kernel.
+template <typename T>
+ses_status enqueue_long_line(const ses_solver* h, int S, bool mask) {
+    const LongEntry<T>* e = reinterpret_cast<const LongEntry<T>*>(h->longk);
+    PassArgs<T> ay = make_args<T>(h, 1, h->psi, h->psi);
+    ay.d_load = DG_HALF;
+    ay.d_mid = DG_FULL;
+    ay.m_mid = mask;
+    ay.d_store = DG_HALF;
+    ay.m_store = mask;
+    const PassArgs<T> ax = make_args<T>(h, 0, h->psi, h->psi);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)e->cs);
+    cfg.blockDim = dim3((unsigned)e->nt);
+    cfg.dynamicSmemBytes = e->smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)e->cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = h->pdl ? 2 : 1;
+    for (int left = S; left > 0; left -= kLineSteps)
+        SES_CU(cudaLaunchKernelEx(&cfg, e->k, ay, ax, std::min(left, kLineSteps)));
+    return SES_OK;
+}
+
 // y/z part of one step: fwd y, fused z, inv y (3D) or fused y (2D) or fused z.
 template <typename T>
 ses_status mid_axes(const ses_solver* h, cudaStream_t s) {
@@ -731,7 +787,7 @@ ses_status interior_unit(const ses_solver* h, bool mask, cudaStream_t s) {
 template <typename T>
 ses_status ensure_body(ses_solver* h, bool mask) {
     cudaGraphExec_t& ex = h->body[mask ? 1 : 0];
-    if (ex || (h->last_axis == 0 && !h->long1d)) return SES_OK;  // 1D lines step in one launch, without a graph
+    if (ex || h->longk || (h->last_axis == 0 && !h->long1d)) return SES_OK;  // lines step in one launch, without a graph
     if (!h->cap) SES_CU(cudaStreamCreateWithFlags(&h->cap, cudaStreamNonBlocking));
     SES_CU(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
     ses_status st = SES_OK;
@@ -755,6 +811,7 @@ ses_status ensure_body(ses_solver* h, bool mask) {
 template <typename T>
 ses_status enqueue_steps(ses_solver* h, int S, bool mask) {
     cudaStream_t s = h->stream;
+    if (h->longk) return enqueue_long_line<T>(h, S, mask);
     if (h->long1d) {
         // [Vh, fwd y, * W] [x: fwd, K/N, inv] {[* conj W, inv y, V (M), fwd y, * W] [x]} ... [* conj W, inv y, Vh (M)]
         XProg first;
@@ -1373,6 +1430,7 @@ template <typename T>
 std::string plan_info_t(const ses_solver* h) {
     std::ostringstream o;
     if (h->long1d) o << "line of " << h->N << " as " << h->n[0] << " x " << h->n[1] << " (four-step): ";
+    if (h->longk) o << "steps on one cluster of " << reinterpret_cast<const LongEntry<T>*>(h->longk)->cs << " CTAs; ";
     const char* names[3] = {"x", "y", "z"};
     for (int a = 0; a < 3; ++a) {
         o << names[a] << ":" << h->n[a];
@@ -1732,6 +1790,7 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     build_tmaps(h, 0, h->psi);
     build_tmaps(h, 1, h->scratch);
     apply_selection(h);
+    h->longk = prec == SES_C128 ? find_long<double>(h) : find_long<float>(h);
     if (with_tables) {
         if ((st = dalloc(h, (void**)&h->V, N * sizeof(double))) != SES_OK) return bail(st);
         if ((st = dalloc(h, &h->vtab, N * h->esize)) != SES_OK) return bail(st);
