@@ -286,8 +286,8 @@ struct ses_solver {
     bool pdl = true;  // single-field passes launched with programmatic stream serialization
     long long wait_limit = 0;      // failure-detection hook: bounded-wait limit of pipelined passes (0: ~2 s)
     uint32_t extra_tx = 0;         // failure-detection hook: bytes each tile barrier expects beyond its copies
-    int xsel = 0;                  // pipelined contiguous-pass variant (-1: register path)
-    int ssel[3] = {0, 0, 0};       // pipelined strided-pass variant per axis (-1: register path)
+    int xsel = -1;                 // pipelined contiguous-pass variant (-1: register path, kXStaged: staged rows)
+    int ssel[3] = {-1, -1, -1};    // pipelined strided-pass variant per axis (-1: register path)
     // two-sweep 3D step (plane pass with the y transforms, then the z pass) when
     // the x-y plane fits in shared memory: the compiled plane pass (nullptr: not
     // available for this grid) and whether steps use it
@@ -538,7 +538,11 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
         const int tl = n / e->e;
         bool done = false;
         const int xs = h->xsel, ss = h->ssel[axis];
-        if (h->pipelined && axis == 0 && xs >= 0 && xs < (int)e->xv.size() && e->xv[xs].k[mode] &&
+        if (h->pipelined && axis == 0 && xs == kXStaged && e->xs[mode] && e->xs_bps[mode] > 0) {
+            const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps[mode]));
+            launch_pass(h->pdl, e->xs[mode], grid, pp.cblock, e->xbsm, s, a, (uint32_t)pp.cgrid);
+            done = true;
+        } else if (h->pipelined && axis == 0 && xs >= 0 && xs < (int)e->xv.size() && e->xv[xs].k[mode] &&
             e->xv[xs].bps[mode] > 0) {
             const auto& v = e->xv[xs];
             PipeArgs pa{};
@@ -1292,8 +1296,21 @@ bool has_planes(const ses_solver* h) {
     return h->prec == SES_C128 ? !handle_planes<double>(h).empty() : !handle_planes<float>(h).empty();
 }
 
-// Selections at creation: cache, then environment overrides SES_XVAR / SES_SVAR / SES_PLANE.
+// The measured default variants of the axes' plans.
+template <typename T>
+void default_variants(ses_solver* h) {
+    for (int a = 0; a < 3; ++a) {
+        const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[a].cp);
+        if (!e) continue;
+        if (a == 0) h->xsel = e->xdef;
+        else h->ssel[a] = a == h->last_axis ? e->fdef : e->sdef;
+    }
+}
+
+// Selections at creation: defaults, cache, then environment overrides SES_XVAR / SES_SVAR / SES_PLANE.
 void apply_selection(ses_solver* h) {
+    if (h->prec == SES_C128) default_variants<double>(h);
+    else default_variants<float>(h);
     apply_plane_choice(h, h->prec == SES_C128 ? default_plane_cs<double>(h) : default_plane_cs<float>(h));
     const std::map<std::string, int> cache = read_tune_cache();
     for (int a = 0; a < 3; ++a) {
@@ -1388,7 +1405,10 @@ ses_status autotune_impl(ses_solver* h, int flags) {
         const int nv = variant_count<T>(h, axis);
         int best = -1;
         float best_ms = 1e30f;
-        for (int c = -1; c < nv; ++c) {
+        std::vector<int> variants;
+        for (int c = -1; c < nv; ++c) variants.push_back(c);
+        if (axis == 0 && h->last_axis > 0) variants.push_back(kXStaged);
+        for (int c : variants) {
             if (axis == 0) h->xsel = c;
             else h->ssel[axis] = c;
             float ms = 0.f;
@@ -1446,7 +1466,9 @@ std::string plan_info_t(const ses_solver* h) {
             o << " E=" << e->e;
             const int sel = a == 0 ? h->xsel : h->ssel[a];
             const int nv = a == 0 ? (int)e->xv.size() : (int)e->sv.size();
-            if (!h->pipelined || sel < 0 || sel >= nv) {
+            if (h->pipelined && a == 0 && sel == kXStaged) {
+                o << " staged rows";
+            } else if (!h->pipelined || sel < 0 || sel >= nv) {
                 o << " register-path";
             } else if (a == 0) {
                 o << " pipelined warps=" << e->xv[sel].warps << " ring=" << e->xv[sel].nbuf << " (variant "
@@ -2078,7 +2100,7 @@ bool svar_ok(const BatchClass& c, int q, int k, int buf) {
 }
 
 // Variant per class pass: the batch's autotuned choice, else the on-disk cache,
-// else the first member's selection; -1 = register-path batched kernel.
+// else the plan's measured default; -1 = register-path batched kernel.
 template <typename T>
 void class_select(const ses_batch_s* b, BatchClass& c) {
     const ses_solver* h0 = c.mem[0];
@@ -2094,10 +2116,11 @@ void class_select(const ses_batch_s* b, BatchClass& c) {
         if (jt != cache.end()) return jt->second;
         return fallback;
     };
-    const int xs = pick(0, h0->xsel);
+    const int xs = pick(0, -1);  // the staged rows of the register path were fastest for every length
     if (xvar_ok<T>(c, xs)) c.xvar = xs;
     for (int q = 0; q < c.nmid; ++q) {
-        const int ss = pick(1 + q, h0->ssel[c.mid_axis[q]]);
+        const auto* e = reinterpret_cast<const PlanEntry<T>*>(h0->pp[c.mid_axis[q]].cp);
+        const int ss = pick(1 + q, !e ? -1 : (c.mid_mode[q] == SM_FUSED ? e->bfdef : e->bsdef));
         if (svar_ok<T>(c, q, ss, 0)) c.svar[q] = ss;
     }
 }

@@ -633,6 +633,37 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     }
 }
 
+// The same for one field (mode START, MID or END): CTAs walk its line tiles with the
+// stage twiddles in shared memory and each tile's potential rows and absorber profile
+// fetched by cp.async while its first transform runs.  Bound by issue and latency (80 us
+// for the 403 MB of a 256^3 complex64 pass, whose copy takes 61).  Between steps, n^3
+// fields, us, TMA-fed or register path -> staged rows: complex64 128 18.7 -> 16.5, 256
+// 93.1 -> 80.6, 512 857 -> 709; complex128 64 9.6 -> 8.3, 128 27.8 -> 22.6, 256 159 -> 132.
+template <typename T, int MODE, int N, int E, int R0, int R1, int R2>
+__global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MINB)
+    xstage_kernel(const __grid_constant__ PassArgs<T> a, const uint32_t tiles) {
+    using XS = XShape<T, N, E>;
+    using TW = TwStage<T, R0, R1, R2>;
+    __shared__ cx<T> xb[XS::NW * XS::LPW * XS::PITCH];
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T>* tw = reinterpret_cast<cx<T>*>(smraw);
+    cx<T>* vt = reinterpret_cast<cx<T>*>(smraw + TW::bytes);
+    TW::load(tw, a.stw, a.stwl);  // a handle's constant table: no need to wait for the previous pass
+    pdl_wait();
+    __syncthreads();
+    const bool fast = MODE == XM_MID && a.d_mid == DG_FULL && a.m_mid && a.tb.maskfull == nullptr &&
+                      a.tb.mask1[0] != nullptr;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        if constexpr (MODE == XM_MID) {
+            if (fast) {
+                xpass2_body<T, MODE, N, E, R0, R1, R2, true, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+                continue;
+            }
+        }
+        xpass2_body<T, MODE, N, E, R0, R1, R2, false, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+    }
+}
+
 // Dynamic shared memory of xbatch_kernel: stage twiddles, then NW * LPW table
 // rows (pitch RPITCH), then one x profile of the absorber (N doubles) per warp.
 template <typename T, int N, int E, int R0, int R1, int R2>

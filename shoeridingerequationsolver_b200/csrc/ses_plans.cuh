@@ -13,6 +13,8 @@ namespace sesk {
 template <typename T>
 using PassKernel = void (*)(const PassArgs<T>);
 
+constexpr int kXStaged = 64;  // contiguous-pass selection: the staged-rows kernel
+
 template <typename T>
 struct PlanEntry {
     int n = 0, e = 0, r0 = 1, r1 = 1, r2 = 1;
@@ -48,6 +50,14 @@ struct PlanEntry {
     };
     std::vector<XVar> xv;
     std::vector<SVar> sv;
+    // contiguous passes of one field on staged rows (xstage_kernel), by XMode
+    using XStage = void (*)(const PassArgs<T>, uint32_t);
+    XStage xs[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    int xs_bps[7] = {0, 0, 0, 0, 0, 0, 0};
+    // default variants (a pipelined variant's index, -1 the register path, x: kXStaged),
+    // as measured: contiguous passes, strided passes, strided passes with the kinetic
+    // phase, and the strided ones of batches
+    int xdef = kXStaged, sdef = -1, fdef = -1, bsdef = -1, bfdef = -1;
     // batched kernels (many fields of this length per launch), by mode
     using XBatch = void (*)(const PassArgs<T>*, const BatchWork);
     XBatch xb[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -99,6 +109,14 @@ PlanEntry<T> make_plan_entry() {
     p.sb[SM_TW_START] = sbatch_kernel<T, SM_TW_START, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_MID] = sbatch_kernel<T, SM_TW_MID, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_END] = sbatch_kernel<T, SM_TW_END, N, E, R0, R1, R2, LS>;
+    p.xs[XM_START] = xstage_kernel<T, XM_START, N, E, R0, R1, R2>;
+    p.xs[XM_MID] = xstage_kernel<T, XM_MID, N, E, R0, R1, R2>;
+    p.xs[XM_END] = xstage_kernel<T, XM_END, N, E, R0, R1, R2>;
+    for (int m : {XM_START, XM_MID, XM_END}) {
+        allow_smem(p.xs[m], (int)p.xbsm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps[m], p.xs[m], p.xw * 32, p.xbsm,
+                                                              cudaOccupancyDefault);
+    }
     for (int m = 0; m < 7; ++m)
         if (p.xb[m]) {
             allow_smem(p.xb[m], (int)p.xbsm);
@@ -181,6 +199,16 @@ void add_s_variant(PlanEntry<T>& p) {
     }
     cudaGetLastError();
     p.sv.push_back(v);
+}
+
+// The measured defaults of an entry: x, strided, fused; batches: strided, fused.
+template <typename T>
+void set_defaults(PlanEntry<T>& p, int x, int s, int f, int bs, int bf) {
+    p.xdef = x;
+    p.sdef = s;
+    p.fdef = f;
+    p.bsdef = bs;
+    p.bfdef = bf;
 }
 
 // defined in ses_plans_*.cu

@@ -13,6 +13,7 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<float, 256, 16, 16, 16, 1, 16, 2, 2>(f.back());
     add_s_variant<float, 256, 16, 16, 16, 1, 16, 3, 2>(f.back());
     add_s_variant<float, 256, 16, 16, 16, 1, 8, 2, 4>(f.back());
+    set_defaults(f.back(), kXStaged, 1, 3, 1, 3);
     d.push_back(make_plan_entry<double, 256, 16, 16, 16, 1, 16>());
     add_x_variant<double, 256, 16, 16, 16, 1, 2, 2, 1>(d.back());
     add_x_variant<double, 256, 16, 16, 16, 1, 4, 2, 2>(d.back());
@@ -20,5 +21,6 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<double, 256, 16, 16, 16, 1, 16, 2, 1>(d.back());
     add_s_variant<double, 256, 16, 16, 16, 1, 8, 2, 2>(d.back());
     add_s_variant<double, 256, 16, 16, 16, 1, 4, 2, 4>(d.back());
+    set_defaults(d.back(), kXStaged, 1, 1, -1, -1);
 }
 }  // namespace sesk

@@ -14,14 +14,17 @@ void register_plans_large(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     f.back().kinds = 2;
     add_s_variant<float, 512, 32, 16, 32, 1, 8, 2, 2>(f.back());
     add_s_variant<float, 512, 32, 16, 32, 1, 4, 2, 4>(f.back());
+    set_defaults(f.back(), kXStaged, 0, 0, 0, 0);
     d.push_back(make_plan_entry<double, 512, 16, 8, 8, 8, 8>());
     add_x_variant<double, 512, 16, 8, 8, 8, 2, 2, 1>(d.back());
     add_s_variant<double, 512, 16, 8, 8, 8, 8, 2, 1>(d.back());
+    set_defaults(d.back(), kXStaged, 0, 0, -1, -1);
     f.push_back(make_plan_entry<float, 1024, 32, 16, 8, 8, 8>());
     f.back().kinds = 1;
     // complex64 1024 strided passes (the y pass of 1024^2 planes): 32x32, two stages
     f.push_back(make_plan_entry<float, 1024, 32, 32, 32, 1, 4>());
     f.back().kinds = 2;
     add_s_variant<float, 1024, 32, 32, 32, 1, 4, 2, 2>(f.back());
+    set_defaults(f.back(), kXStaged, 0, 0, 0, 0);
 }
 }  // namespace sesk

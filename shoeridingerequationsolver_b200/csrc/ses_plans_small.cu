@@ -10,19 +10,23 @@ void register_plans_small(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     add_x_variant<float, 32, 8, 8, 4, 1, 8, 2, 2>(f.back());
     add_s_variant<float, 32, 8, 8, 4, 1, 32, 2, 4>(f.back());
     add_s_variant<float, 32, 8, 8, 4, 1, 32, 3, 3>(f.back());
+    set_defaults(f.back(), kXStaged, 0, 0, 0, 0);
     d.push_back(make_plan_entry<double, 32, 8, 8, 4, 1, 16>());
     f.push_back(make_plan_entry<float, 64, 8, 8, 8, 1, 32>());
     add_x_variant<float, 64, 8, 8, 8, 1, 4, 2, 2>(f.back());
     add_s_variant<float, 64, 8, 8, 8, 1, 32, 2, 2>(f.back());
+    set_defaults(f.back(), kXStaged, -1, 0, 0, 0);
     d.push_back(make_plan_entry<double, 64, 8, 8, 8, 1, 16>());
     add_x_variant<double, 64, 8, 8, 8, 1, 4, 2, 2>(d.back());
     add_s_variant<double, 64, 8, 8, 8, 1, 16, 2, 2>(d.back());
+    set_defaults(d.back(), kXStaged, -1, 0, -1, -1);
     f.push_back(make_plan_entry<float, 128, 16, 16, 8, 1, 32>());
     add_x_variant<float, 128, 16, 16, 8, 1, 4, 2, 3>(f.back());
     add_x_variant<float, 128, 16, 16, 8, 1, 2, 2, 6>(f.back());
     add_s_variant<float, 128, 16, 16, 8, 1, 32, 2, 1>(f.back());
     add_s_variant<float, 128, 16, 16, 8, 1, 16, 2, 2>(f.back());
     add_s_variant<float, 128, 16, 16, 8, 1, 8, 2, 4>(f.back());
+    set_defaults(f.back(), kXStaged, -1, 1, 1, 1);
     d.push_back(make_plan_entry<double, 128, 16, 16, 8, 1, 16>());
 }
 }  // namespace sesk
