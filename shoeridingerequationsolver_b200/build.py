@@ -20,7 +20,7 @@ LIB = PKG / "libses_b200.so"
 SOURCES = ["ses_gpu.cu", "ses_plans_small.cu", "ses_plans_mixed.cu", "ses_plans_256.cu",
            "ses_plans_large.cu", "ses_plans_plane.cu", "ses_line_c64.cu", "ses_line_c128.cu", "ses_longline.cu",
            "ses_noalloc.cu", "ses_serve.cpp"]
-HEADERS = ["ses_fft.cuh", "ses_pass.cuh", "ses_pass2.cuh", "ses_pass3.cuh", "ses_tma.cuh", "ses_plans.cuh", "ses_engine.cuh",
+HEADERS = ["ses_fft.cuh", "ses_pass.cuh", "ses_pass2.cuh", "ses_pass3.cuh", "ses_pass4.cuh", "ses_tma.cuh", "ses_plans.cuh", "ses_engine.cuh",
            "ses_aux.cuh", "ses_plane.cuh", "ses_line.cuh", "ses_line_inst.cuh",
            "ses_longline.cuh"]
 

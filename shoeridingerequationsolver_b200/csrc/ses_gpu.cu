@@ -277,7 +277,7 @@ struct ses_solver {
     size_t bytes = 0;
 
     // pipelined passes: TMA descriptors of psi / scratch along y and z, per variant
-    static constexpr int kMaxVar = 4;
+    static constexpr int kMaxVar = 8;
     CUtensorMap tmap[2][3][kMaxVar];
     bool tmap_ok[2][3][kMaxVar] = {};
     unsigned* herr = nullptr;  // error word (page-locked) that the device's bounded waits set
@@ -535,7 +535,6 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
     {
         const PlanEntry<T>* e = reinterpret_cast<const PlanEntry<T>*>(pp.cp);
         const int n = h->n[axis];
-        const int tl = n / e->e;
         bool done = false;
         const int xs = h->xsel, ss = h->ssel[axis];
         if (h->pipelined && axis == 0 && xs == kXStaged && e->xs[mode] && e->xs_bps[mode] > 0) {
@@ -569,7 +568,7 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
                 pa.wait_limit = h->wait_limit;
                 pa.extra_tx = h->extra_tx;
                 const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
-                launch_pass(h->pdl, v.k[mode], (unsigned)grid, (unsigned)(v.ls * tl), v.smem, s, a,
+                launch_pass(h->pdl, v.k[mode], (unsigned)grid, (unsigned)v.threads, v.smem, s, a,
                             h->tmap[buf][axis][ss], pa);
                 done = true;
             }
@@ -1474,7 +1473,7 @@ std::string plan_info_t(const ses_solver* h) {
                 o << " pipelined warps=" << e->xv[sel].warps << " ring=" << e->xv[sel].nbuf << " (variant "
                   << sel << ")";
             } else {
-                o << " pipelined TMA lines=" << e->sv[sel].ls << " ring=" << e->sv[sel].nbuf << " (variant "
+                o << (e->sv[sel].swizzle ? " pipelined TMA warp lines=" : " pipelined TMA lines=") << e->sv[sel].ls << " ring=" << e->sv[sel].nbuf << " (variant "
                   << sel << ")";
             }
         }
@@ -1642,6 +1641,9 @@ void build_tmaps_t(ses_solver* h, int buf, void* base, EncodeTiledFn enc) {
         const cuuint64_t nx = h->n[0], ny = h->n[1], nz = h->n[2];
         for (int k = 0; k < (int)e->sv.size() && k < ses_solver::kMaxVar; ++k) {
             const int ls = e->sv[k].ls;
+            const CUtensorMapSwizzle swz = e->sv[k].swizzle == 64    ? CU_TENSOR_MAP_SWIZZLE_64B
+                                           : e->sv[k].swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                                                     : CU_TENSOR_MAP_SWIZZLE_NONE;
             CUresult r;
             if (axis == 1) {
                 if (nx % (cuuint64_t)ls) continue;  // a tile must not cross z
@@ -1650,7 +1652,7 @@ void build_tmaps_t(ses_solver* h, int buf, void* base, EncodeTiledFn enc) {
                 const cuuint32_t box[3] = {(cuuint32_t)(ls * ew), rows, 1};
                 const cuuint32_t es[3] = {1, 1, 1};
                 r = enc(&h->tmap[buf][axis][k], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             } else {
                 const cuuint64_t dims[2] = {nx * ny * ew, nz};
@@ -1658,7 +1660,7 @@ void build_tmaps_t(ses_solver* h, int buf, void* base, EncodeTiledFn enc) {
                 const cuuint32_t box[2] = {(cuuint32_t)(ls * ew), rows};
                 const cuuint32_t es[2] = {1, 1};
                 r = enc(&h->tmap[buf][axis][k], CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             }
             h->tmap_ok[buf][axis][k] = (r == CUDA_SUCCESS);
@@ -2397,7 +2399,7 @@ ses_status class_launch(const ses_batch_s* b, const BatchClass& c, int prog, boo
         } else {
             const auto& v = e->sv[c.svar[q]];
             const unsigned grid = std::min<unsigned>(w.total, (unsigned)(b->sms * v.bbps[mode]));
-            launch_pass(h0->pdl, v.kb[mode], grid, (unsigned)(v.ls * (n / e->e)), v.smem, s, args,
+            launch_pass(h0->pdl, v.kb[mode], grid, (unsigned)v.threads, v.smem, s, args,
                         maps + (size_t)q * nm, w, pa);
         }
         const cudaError_t err = cudaGetLastError();

@@ -7,6 +7,7 @@
 
 #include "ses_pass2.cuh"
 #include "ses_pass3.cuh"
+#include "ses_pass4.cuh"
 
 namespace sesk {
 
@@ -44,6 +45,8 @@ struct PlanEntry {
         SPipe k[kSModes] = {};
         SBPipe kb[kSModes] = {};
         int ls = 0, nbuf = 0;
+        int threads = 0;
+        int swizzle = 0;  // bytes of a swizzled tile row (ses_pass4.cuh), 0: plain rows
         size_t smem = 0;
         int bps[kSModes] = {};
         int bbps[kSModes] = {};
@@ -178,6 +181,7 @@ void add_s_variant(PlanEntry<T>& p) {
     typename PlanEntry<T>::SVar v;
     v.ls = LS;
     v.nbuf = NBUF;
+    v.threads = LS * TL;
     v.k[SM_FWD] = spass3_kernel<T, SM_FWD, N, E, R0, R1, R2, LS, NBUF, MINB>;
     v.k[SM_INV] = spass3_kernel<T, SM_INV, N, E, R0, R1, R2, LS, NBUF, MINB>;
     v.k[SM_FUSED] = spass3_kernel<T, SM_FUSED, N, E, R0, R1, R2, LS, NBUF, MINB>;
@@ -196,6 +200,34 @@ void add_s_variant(PlanEntry<T>& p) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&v.bbps[m], v.kb[m], LS * TL, v.smem,
                                                                   cudaOccupancyDefault);
         }
+    }
+    cudaGetLastError();
+    p.sv.push_back(v);
+}
+
+// Variant with warp-owned lines (ses_pass4.cuh): tile rows of RB bytes, NG groups of
+// warps, NBUF tiles.
+template <typename T, int N, int E, int R0, int R1, int RB, int NG, int NBUF>
+void add_s4_variant(PlanEntry<T>& p) {
+    using P = Pass4Shape<T, N, E, R0, R1, RB, NG, NBUF>;
+    typename PlanEntry<T>::SVar v;
+    v.ls = P::L;
+    v.nbuf = NBUF;
+    v.threads = P::NT;
+    v.swizzle = RB;
+    v.smem = P::smem;
+    v.k[SM_FWD] = spass4_kernel<T, SM_FWD, N, E, R0, R1, RB, NG, NBUF>;
+    v.k[SM_INV] = spass4_kernel<T, SM_INV, N, E, R0, R1, RB, NG, NBUF>;
+    v.k[SM_FUSED] = spass4_kernel<T, SM_FUSED, N, E, R0, R1, RB, NG, NBUF>;
+    v.kb[SM_FWD] = sbatch4_kernel<T, SM_FWD, N, E, R0, R1, RB, NG, NBUF>;
+    v.kb[SM_INV] = sbatch4_kernel<T, SM_INV, N, E, R0, R1, RB, NG, NBUF>;
+    v.kb[SM_FUSED] = sbatch4_kernel<T, SM_FUSED, N, E, R0, R1, RB, NG, NBUF>;
+    for (int m : {SM_FWD, SM_INV, SM_FUSED}) {
+        allow_smem(v.k[m], (int)v.smem);
+        allow_smem(v.kb[m], (int)v.smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&v.bps[m], v.k[m], v.threads, v.smem, cudaOccupancyDefault);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&v.bbps[m], v.kb[m], v.threads, v.smem,
+                                                              cudaOccupancyDefault);
     }
     cudaGetLastError();
     p.sv.push_back(v);

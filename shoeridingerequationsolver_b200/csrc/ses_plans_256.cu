@@ -13,7 +13,8 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<float, 256, 16, 16, 16, 1, 16, 2, 2>(f.back());
     add_s_variant<float, 256, 16, 16, 16, 1, 16, 3, 2>(f.back());
     add_s_variant<float, 256, 16, 16, 16, 1, 8, 2, 4>(f.back());
-    set_defaults(f.back(), kXStaged, 1, 3, 1, 3);
+    add_s4_variant<float, 256, 16, 16, 16, 64, 4, 12>(f.back());
+    set_defaults(f.back(), kXStaged, 4, 4, 4, 4);
     d.push_back(make_plan_entry<double, 256, 16, 16, 16, 1, 16>());
     add_x_variant<double, 256, 16, 16, 16, 1, 2, 2, 1>(d.back());
     add_x_variant<double, 256, 16, 16, 16, 1, 4, 2, 2>(d.back());
@@ -21,6 +22,7 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<double, 256, 16, 16, 16, 1, 16, 2, 1>(d.back());
     add_s_variant<double, 256, 16, 16, 16, 1, 8, 2, 2>(d.back());
     add_s_variant<double, 256, 16, 16, 16, 1, 4, 2, 4>(d.back());
-    set_defaults(d.back(), kXStaged, 1, 1, -1, -1);
+    add_s4_variant<double, 256, 16, 16, 16, 64, 6, 12>(d.back());
+    set_defaults(d.back(), kXStaged, 3, 3, 3, 3);
 }
 }  // namespace sesk

@@ -14,7 +14,8 @@ void register_plans_large(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     f.back().kinds = 2;
     add_s_variant<float, 512, 32, 16, 32, 1, 8, 2, 2>(f.back());
     add_s_variant<float, 512, 32, 16, 32, 1, 4, 2, 4>(f.back());
-    set_defaults(f.back(), kXStaged, 0, 0, 0, 0);
+    add_s4_variant<float, 512, 32, 16, 32, 64, 2, 6>(f.back());
+    set_defaults(f.back(), kXStaged, 0, 2, 0, 2);
     d.push_back(make_plan_entry<double, 512, 16, 8, 8, 8, 8>());
     add_x_variant<double, 512, 16, 8, 8, 8, 2, 2, 1>(d.back());
     add_s_variant<double, 512, 16, 8, 8, 8, 8, 2, 1>(d.back());

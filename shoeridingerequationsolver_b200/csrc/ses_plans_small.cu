@@ -15,10 +15,12 @@ void register_plans_small(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     f.push_back(make_plan_entry<float, 64, 8, 8, 8, 1, 32>());
     add_x_variant<float, 64, 8, 8, 8, 1, 4, 2, 2>(f.back());
     add_s_variant<float, 64, 8, 8, 8, 1, 32, 2, 2>(f.back());
-    set_defaults(f.back(), kXStaged, -1, 0, 0, 0);
+    add_s4_variant<float, 64, 8, 8, 8, 128, 4, 16>(f.back());
+    set_defaults(f.back(), kXStaged, -1, 0, 0, 1);
     d.push_back(make_plan_entry<double, 64, 8, 8, 8, 1, 16>());
     add_x_variant<double, 64, 8, 8, 8, 1, 4, 2, 2>(d.back());
     add_s_variant<double, 64, 8, 8, 8, 1, 16, 2, 2>(d.back());
+    add_s4_variant<double, 64, 8, 8, 8, 128, 6, 18>(d.back());
     set_defaults(d.back(), kXStaged, -1, 0, -1, -1);
     f.push_back(make_plan_entry<float, 128, 16, 16, 8, 1, 32>());
     add_x_variant<float, 128, 16, 16, 8, 1, 4, 2, 3>(f.back());
@@ -26,7 +28,10 @@ void register_plans_small(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     add_s_variant<float, 128, 16, 16, 8, 1, 32, 2, 1>(f.back());
     add_s_variant<float, 128, 16, 16, 8, 1, 16, 2, 2>(f.back());
     add_s_variant<float, 128, 16, 16, 8, 1, 8, 2, 4>(f.back());
-    set_defaults(f.back(), kXStaged, -1, 1, 1, 1);
+    add_s4_variant<float, 128, 16, 16, 8, 128, 4, 12>(f.back());
+    set_defaults(f.back(), kXStaged, -1, 3, 3, 3);
     d.push_back(make_plan_entry<double, 128, 16, 16, 8, 1, 16>());
+    add_s4_variant<double, 128, 16, 16, 8, 128, 6, 12>(d.back());
+    set_defaults(d.back(), kXStaged, 0, 0, 0, 0);
 }
 }  // namespace sesk
