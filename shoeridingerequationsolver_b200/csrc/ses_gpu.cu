@@ -1265,16 +1265,19 @@ bool select_plane(ses_solver* h, int cs) {
 }
 
 // Default step form of a grid with plane passes, from B200 measurements of
-// single-handle n^3 steps (us per step: four axis passes / plane on 1 CTA / on a
-// cluster of 2): complex128 32: 8.2 / 6.9 / 7.7, 48: 12.6 / 12.8 / 11.8,
-// 64: 14.6 / 13.1 / 11.8 (the one-CTA plane leaves 84 of 148 SMs idle on 64
-// planes); complex64 32: 9.7 / 5.9 / 7.4, 48: 12.8 / 8.5 / 9.7, 64: 12.8 / 10.5 /
-// 10.3, 96: 25.9 / 21.5 / 22.6, 128: 47.1 / 36.4 / --.
+// single-handle n^3 steps with an absorber (us per step: four axis passes / plane on
+// 1 CTA / on a cluster of 2 / of 4): complex64 32: 9.6 / 6.5 / 7.7 / --, 48: 10.8 /
+// 8.2 / 9.5 / --, 64: 11.5 / 10.6 / 9.8 / 10.2, 96: 20.8 / 21.6 / 22.2 / 22.1, 128:
+// 37.5 / 32.1 / --; complex128 32: 9.0 / 7.0 / 7.7 / --, 48: 13.4 / 13.1 / 11.8 / --,
+// 64: 12.9 / 13.1 / 11.4 / 11.6.
 template <typename T>
 int default_plane_cs(const ses_solver* h) {
     auto planes = handle_planes<T>(h);
     if (planes.empty()) return 0;
-    const int want = sizeof(T) == 8 && h->n[0] >= 48 ? 2 : 1;
+    const int n = h->n[0];
+    int want = 1;
+    if (sizeof(T) == 8 ? n >= 48 : n == 64) want = 2;
+    if (sizeof(T) == 4 && n == 96) want = 0;
     for (auto* e : planes)
         if (e->cs == want) return want;
     return 0;  // other variants only when the autotuner or SES_PLANE picks them

@@ -166,7 +166,7 @@ struct XchWarp {
 template <int N, int E>
 struct XPad {
     static constexpr bool k160e40 = N == 160 && E == 40;  // plan 20 x 8
-    static constexpr int SH = N == 160 || N == 96 || N == 64 ? 3 : (N == 48 || N == 32 ? 2 : 4);
+    static constexpr int SH = N == 1024 ? 5 : N == 160 || N == 96 || N == 64 ? 3 : (N == 48 || N == 32 ? 2 : 4);
     static constexpr int PM = N == 48 ? 3 : 1;
     static constexpr int LPAD = k160e40 ? 0 : (N == 160 ? 4 : (N == 96 ? 12 : (N == 32 ? 4 : 0)));
     static constexpr int PITCH = N + PM * (N >> SH) + LPAD;
@@ -219,15 +219,24 @@ struct XShape {
 // vt (optional): shared memory for this CTA's potential-table rows (NW * LPW
 // lines of N entries); the between-steps and batch-end passes then fetch the
 // rows asynchronously at the start of the tile and read them after the first FFT.
-// FASTKICK (between-steps pass of the batched kernel only): the pass applies the
-// full kick with a separable absorber from staged table and profile rows -- the
-// run-time tests of the general path (table kind, mask kind, staged rows) are
-// resolved at compile time, leaving straight-line code per element.
-template <typename T, int MODE, int N, int E, int R0, int R1, int R2, bool FASTKICK = false, bool PK = false,
-          class A>
+// KICK (between-steps pass on staged rows only): the pass applies the full kick with a
+// separable absorber (KICK_SEP) or without one (KICK_PLAIN) from staged table and
+// profile rows -- the run-time tests of the general path (table kind, mask kind, staged
+// rows) are resolved at compile time, leaving straight-line code per element.
+enum KickForm : int { KICK_ANY = 0, KICK_SEP = 1, KICK_PLAIN = 2 };
+
+template <typename T>
+__device__ __forceinline__ int kick_form(const PassArgs<T>& a) {  // of a between-steps pass
+    if (a.d_mid != DG_FULL) return KICK_ANY;
+    if (!a.m_mid) return KICK_PLAIN;
+    return a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr ? KICK_SEP : KICK_ANY;
+}
+
+template <typename T, int MODE, int N, int E, int R0, int R1, int R2, int KICK = KICK_ANY, bool PK = false, class A>
 __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb, const cx<T>* twh,
                                             const cx<T>* twl, cx<T>* vt = nullptr) {
-    static_assert(!FASTKICK || MODE == XM_MID, "the fast kick is the between-steps pass");
+    static_assert(KICK == KICK_ANY || MODE == XM_MID, "the straight-line kick is the between-steps pass");
+    constexpr bool FASTKICK = KICK != KICK_ANY;
     using XS = XShape<T, N, E>;
     constexpr int TL = XS::TL;
     constexpr int LPW = XS::LPW;
@@ -275,7 +284,8 @@ __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb
         }
     if constexpr (kTabLate) {
         const bool want = FASTKICK || (MODE == XM_MID ? a.d_mid != DG_NONE : a.d_store != DG_NONE);
-        const bool wantm = FASTKICK || ((MODE == XM_MID ? a.m_mid : a.m_store) && !mfull && mx);
+        const bool wantm =
+            KICK == KICK_SEP || (KICK == KICK_ANY && (MODE == XM_MID ? a.m_mid : a.m_store) && !mfull && mx);
         if (FASTKICK || (vt && (want || wantm))) {  // this warp's rows, 16-byte chunks spread over the lanes
             __syncwarp();  // the previous tile's reads of these rows are done
             if (want) {  // line by line, lane-strided 16-byte chunks: constant offsets per copy
@@ -371,9 +381,11 @@ __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb
             for (int r = 0; r < RL; ++r) {
                 const int pos = q + TL * b + r * (N / RL);
                 cx<T> e = v[b * RL + r];
-                if constexpr (MODE == XM_MID && FASTKICK) {
+                if constexpr (MODE == XM_MID && KICK == KICK_SEP) {
                     // (psi h (m)) h with the staged row h and profile mx, m = mx[pos] my[j] mz[k]
                     e = apply_diag_tv(cconj(e), DG_FULL, vrow[pos], 1, ms[pos] * myz);
+                } else if constexpr (MODE == XM_MID && KICK == KICK_PLAIN) {
+                    e = apply_diag_tv(cconj(e), DG_FULL, vrow[pos], 0, 1.0);
                 } else if constexpr (MODE == XM_MID) {
                     e = cconj(e);
                     if (a.d_mid != DG_NONE || a.m_mid) e = diag(e, a.d_mid, a.m_mid, pos);
@@ -619,17 +631,19 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     for (uint32_t t = blockIdx.x; t < w.total; t += gridDim.x) {
         const uint32_t inst = fdiv(t, w.fbpi);
         const PassArgs<T>& a = args[inst];
-        if constexpr (MODE == XM_MID) {
-            // the common between-steps program: full kick and a separable absorber
-            if (a.d_mid == DG_FULL && a.m_mid && a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, true, true>(a, (long long)(t - inst * w.bpi), xb, tw,
-                                                                   TW::lo_of(tw),
-                                                             vt);
+        const long long tile = (long long)(t - inst * w.bpi);
+        if constexpr (MODE == XM_MID) {  // the common between-steps programs: full kick, separable absorber or none
+            const int form = kick_form(a);
+            if (form == KICK_SEP) {
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
+                continue;
+            }
+            if (form == KICK_PLAIN) {
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_PLAIN, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
                 continue;
             }
         }
-        xpass2_body<T, MODE, N, E, R0, R1, R2, false, true>(a, (long long)(t - inst * w.bpi), xb, tw, TW::lo_of(tw),
-                                                            vt);
+        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
     }
 }
 
@@ -651,16 +665,19 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     TW::load(tw, a.stw, a.stwl);  // a handle's constant table: no need to wait for the previous pass
     pdl_wait();
     __syncthreads();
-    const bool fast = MODE == XM_MID && a.d_mid == DG_FULL && a.m_mid && a.tb.maskfull == nullptr &&
-                      a.tb.mask1[0] != nullptr;
+    const int form = MODE == XM_MID ? kick_form(a) : (int)KICK_ANY;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         if constexpr (MODE == XM_MID) {
-            if (fast) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, true, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+            if (form == KICK_SEP) {
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+                continue;
+            }
+            if (form == KICK_PLAIN) {
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_PLAIN, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
                 continue;
             }
         }
-        xpass2_body<T, MODE, N, E, R0, R1, R2, false, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
     }
 }
 
