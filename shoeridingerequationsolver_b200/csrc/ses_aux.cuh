@@ -153,7 +153,7 @@ __global__ void build_vtab_c64(const double* __restrict__ V, cx<float>* out, lon
 // (blockIdx.y) has the x, y and z factors one after the other, n0 + n1 + n2 of them --
 // a sincos per axis point and kick instead of one per cell.  delta: cis - 1
 // (complex64), without cancellation.
-constexpr int kKicks = 64;  // kicks per launch
+constexpr int kKicks = 16;  // kicks per launch
 struct KickArgs {
     int n[3];
     double axis[3], origin[3], h[3];

@@ -888,7 +888,6 @@ ses_status enqueue_driven(ses_solver* h, int S, bool mask, const double* axis, d
     const double dt = h->dt;
     auto theta = [&](double t) { return amp * std::cos(omega * t) * 0.5 * dt; };
     const int per_kick = h->n[0] + h->n[1] + h->n[2];
-    if (!h->kicks) SES_TRY(dalloc(h, (void**)&h->kicks, (size_t)kKicks * per_kick * sizeof(cx<double>)));
     for (int i = 0; i <= S; ++i) {  // kick i: before step i, between steps i - 1 and i, after the last
         if (i % kKicks == 0) {
             KickArgs a{};
@@ -1818,6 +1817,11 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     build_tmaps(h, 1, h->scratch);
     apply_selection(h);
     h->longk = prec == SES_C128 ? find_long<double>(h) : find_long<float>(h);
+    // here, not at the first driven call, which may be under stream capture
+    if (with_tables && !imag && h->last_axis > 0 && !h->long1d &&
+        (st = dalloc(h, (void**)&h->kicks,
+                     (size_t)kKicks * (h->n[0] + h->n[1] + h->n[2]) * sizeof(cx<double>))) != SES_OK)
+        return bail(st);
     if (with_tables) {
         if ((st = dalloc(h, (void**)&h->V, N * sizeof(double))) != SES_OK) return bail(st);
         if ((st = dalloc(h, &h->vtab, N * h->esize)) != SES_OK) return bail(st);

@@ -185,8 +185,10 @@ __device__ __forceinline__ void spass4_body(const F& f, const PipeArgs& pa) {
             const long long lim = 2 * (pa.wait_limit > 0 ? pa.wait_limit : kWaitLimitCycles);
             if (!mbar_wait(smem_u32(&done[buf]), (uint32_t)((i / NBUF) & 1), lim)) {
                 atomicOr(pa.err, 1u);
-                for (int j = i; j < nmine && j < i + NBUF; ++j)  // drain the loads in flight (bounded)
-                    (void)mbar_wait(smem_u32(&full[j % NBUF]), (uint32_t)((j / NBUF) & 1), pa.wait_limit);
+                // drain the loads in flight, a tile each (bounded: 50 ms is far beyond a load's time)
+                const long long drain = lim < 100000000LL ? lim : 100000000LL;
+                for (int j = i; j < nmine && j < i + NBUF; ++j)
+                    (void)mbar_wait(smem_u32(&full[j % NBUF]), (uint32_t)((j / NBUF) & 1), drain);
                 break;
             }
             const CUtensorMap* map;

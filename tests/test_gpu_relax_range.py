@@ -42,3 +42,19 @@ def test_relax_with_steep_potentials(ses, oracle, prec, tol, offset, nsteps):
         n2 = float(np.sum(np.abs(f) ** 2) * g.cell_volume())
         assert abs(e + math.log(n2) / (2 * dtau)) <= (1e-9 if prec == "c128" else 1e-3) * max(1.0, abs(offset))
     op.close()
+
+
+@pytest.mark.parametrize("prec,tol", [("c128", 1e-12), ("c64", 1e-5)])
+@pytest.mark.parametrize("dims", [(360, 1, 1), (50, 36, 1), (64, 64, 1), (30, 1, 24)])
+def test_relax_on_lines_and_planes(ses, oracle, prec, tol, dims):
+    box = tuple(v for d in dims for v in ((-6.0, 6.0) if d > 1 else (0.0, 1.0)))
+    live = [1.0 if d > 1 else 0.0 for d in dims]
+    V = oracle.harmonic3d(box, dims, 1.0, tuple(0.2 * a for a in live))
+    psi = oracle.gaussian3d(box, dims, tuple(0.6 * a for a in live), (1.2, 0.9, 1.1), (0.0, 0.0, 0.0))
+    g = ses.Grid3D(*(ses.Grid1D(box[2 * a], box[2 * a + 1], dims[a]) for a in range(3)))
+    want = oracle.relax3d(box, dims, V, 0.01, psi, 40)
+    for every in (1, 7):
+        op = ses.ImaginaryTimePropagator3D(g, V, 0.01, precision=prec, psi0=psi)
+        op.relax_resident(40, renorm_every=every)
+        assert rel(op.readback(), want) <= tol, every
+        op.close()

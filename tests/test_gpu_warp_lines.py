@@ -107,3 +107,20 @@ def test_warp_lines_in_batches(ses, oracle, dims, prec, tmp_path, monkeypatch):
                 assert rel(op.readback(), want) < (1e-11 if prec == "c128" else 1e-5), (svar, dt, info)
         for op in ops:
             op.close()
+
+
+def test_expired_wait_in_a_warp_line_pass(ses, oracle):
+    """The failure-detection hook on a warp-line pass: the wait runs out (1 ms, 16 bytes
+    that no copy delivers), the status says so, and the handle steps correctly after."""
+    dims = (16, 16, 256)
+    box, g, V, psi = scene(ses, oracle, dims)
+    op = make(ses, g, V, psi, "c64", 4)
+    op.set_wait_limit(2_000_000, 16)
+    op.advance(2)
+    with pytest.raises(TimeoutError):
+        op.sync(30000)
+    op.set_wait_limit(0, 0)
+    op.upload_state(psi)
+    op.advance(5)
+    assert rel(op.readback(), oracle.step3d(box, dims, V, 0.01, psi, 5)) < 1e-5
+    op.close()
