@@ -539,7 +539,7 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
         const int xs = h->xsel, ss = h->ssel[axis];
         if (h->pipelined && axis == 0 && xs == kXStaged && e->xs[mode] && e->xs_bps[mode] > 0) {
             const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps[mode]));
-            launch_pass(h->pdl, e->xs[mode], grid, pp.cblock, e->xbsm, s, a, (uint32_t)pp.cgrid);
+            launch_pass(h->pdl, e->xs[mode], grid, pp.cblock, e->xssm, s, a, (uint32_t)pp.cgrid);
             done = true;
         } else if (h->pipelined && axis == 0 && xs >= 0 && xs < (int)e->xv.size() && e->xv[xs].k[mode] &&
             e->xv[xs].bps[mode] > 0) {

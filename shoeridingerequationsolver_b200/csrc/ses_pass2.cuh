@@ -232,9 +232,11 @@ __device__ __forceinline__ int kick_form(const PassArgs<T>& a) {  // of a betwee
     return a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr ? KICK_SEP : KICK_ANY;
 }
 
-template <typename T, int MODE, int N, int E, int R0, int R1, int R2, int KICK = KICK_ANY, bool PK = false, class A>
+// MPRE: mpre holds the x profile of a separable absorber, staged once for all tiles.
+template <typename T, int MODE, int N, int E, int R0, int R1, int R2, int KICK = KICK_ANY, bool PK = false,
+          bool MPRE = false, class A>
 __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb, const cx<T>* twh,
-                                            const cx<T>* twl, cx<T>* vt = nullptr) {
+                                            const cx<T>* twl, cx<T>* vt = nullptr, double* mpre = nullptr) {
     static_assert(KICK == KICK_ANY || MODE == XM_MID, "the straight-line kick is the between-steps pass");
     constexpr bool FASTKICK = KICK != KICK_ANY;
     using XS = XShape<T, N, E>;
@@ -267,7 +269,8 @@ __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb
     const double* mx = a.tb.mask1[0];
     // this warp's copy of the x profile of a separable absorber (N doubles after the
     // table rows of all warps), staged with the rows by the passes that use it
-    double* ms = vt ? reinterpret_cast<double*>(vt + (size_t)NW * LPW * RP) + (size_t)warp * N : nullptr;
+    double* ms = MPRE ? mpre
+                      : (vt ? reinterpret_cast<double*>(vt + (size_t)NW * LPW * RP) + (size_t)warp * N : nullptr);
     // load the first FFT's inputs (coalesced along the line)
     constexpr bool kConjIn = MODE == XM_INV || MODE == XM_MID || MODE == XM_END;
 #pragma unroll
@@ -285,7 +288,7 @@ __device__ __forceinline__ void xpass2_body(const A& a, long long blk, cx<T>* xb
     if constexpr (kTabLate) {
         const bool want = FASTKICK || (MODE == XM_MID ? a.d_mid != DG_NONE : a.d_store != DG_NONE);
         const bool wantm =
-            KICK == KICK_SEP || (KICK == KICK_ANY && (MODE == XM_MID ? a.m_mid : a.m_store) && !mfull && mx);
+            !MPRE && (KICK == KICK_SEP || (KICK == KICK_ANY && (MODE == XM_MID ? a.m_mid : a.m_store) && !mfull && mx));
         if (FASTKICK || (vt && (want || wantm))) {  // this warp's rows, 16-byte chunks spread over the lanes
             __syncwarp();  // the previous tile's reads of these rows are done
             if (want) {  // line by line, lane-strided 16-byte chunks: constant offsets per copy
@@ -652,7 +655,17 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
 // fetched by cp.async while its first transform runs.  Bound by issue and latency (80 us
 // for the 403 MB of a 256^3 complex64 pass, whose copy takes 61).  Between steps, n^3
 // fields, us, TMA-fed or register path -> staged rows: complex64 128 18.7 -> 16.5, 256
-// 93.1 -> 80.6, 512 857 -> 709; complex128 64 9.6 -> 8.3, 128 27.8 -> 22.6, 256 159 -> 132.
+// 93.1 -> 80.6, 512 857 -> 678; complex128 64 9.6 -> 8.3, 128 27.8 -> 22.6, 256 159 -> 132.
+// The absorber's x profile is one field's, so a CTA stages it once: with a copy per warp
+// and tile it took a third of the staged bytes and, at 512 points, a CTA of the SM
+// (512^3 pass 709 -> 678 us; 1024^2 step 28.0 -> 22.6).
+template <typename T, int N, int E, int R0, int R1, int R2>
+constexpr size_t xstage_smem() {
+    return TwStage<T, R0, R1, R2>::bytes +
+           (size_t)XShape<T, N, E>::NW * XShape<T, N, E>::LPW * XShape<T, N, E>::RPITCH * sizeof(cx<T>) +
+           (size_t)N * sizeof(double);
+}
+
 template <typename T, int MODE, int N, int E, int R0, int R1, int R2>
 __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MINB)
     xstage_kernel(const __grid_constant__ PassArgs<T> a, const uint32_t tiles) {
@@ -662,22 +675,26 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* tw = reinterpret_cast<cx<T>*>(smraw);
     cx<T>* vt = reinterpret_cast<cx<T>*>(smraw + TW::bytes);
+    double* mrow = reinterpret_cast<double*>(vt + (size_t)XS::NW * XS::LPW * XS::RPITCH);
     TW::load(tw, a.stw, a.stwl);  // a handle's constant table: no need to wait for the previous pass
     pdl_wait();
+    if (a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr)
+        for (int i = threadIdx.x; i < N; i += blockDim.x) mrow[i] = a.tb.mask1[0][i];
     __syncthreads();
     const int form = MODE == XM_MID ? kick_form(a) : (int)KICK_ANY;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const long long tile = (long long)t;
         if constexpr (MODE == XM_MID) {
             if (form == KICK_SEP) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
                 continue;
             }
             if (form == KICK_PLAIN) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_PLAIN, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_PLAIN, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
                 continue;
             }
         }
-        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt);
+        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
     }
 }
 

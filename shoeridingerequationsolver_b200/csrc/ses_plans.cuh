@@ -57,6 +57,7 @@ struct PlanEntry {
     using XStage = void (*)(const PassArgs<T>, uint32_t);
     XStage xs[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     int xs_bps[7] = {0, 0, 0, 0, 0, 0, 0};
+    size_t xssm = 0;
     // default variants (a pipelined variant's index, -1 the register path, x: kXStaged),
     // as measured: contiguous passes, strided passes, strided passes with the kinetic
     // phase, and the strided ones of batches
@@ -112,12 +113,13 @@ PlanEntry<T> make_plan_entry() {
     p.sb[SM_TW_START] = sbatch_kernel<T, SM_TW_START, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_MID] = sbatch_kernel<T, SM_TW_MID, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_END] = sbatch_kernel<T, SM_TW_END, N, E, R0, R1, R2, LS>;
+    p.xssm = xstage_smem<T, N, E, R0, R1, R2>();
     p.xs[XM_START] = xstage_kernel<T, XM_START, N, E, R0, R1, R2>;
     p.xs[XM_MID] = xstage_kernel<T, XM_MID, N, E, R0, R1, R2>;
     p.xs[XM_END] = xstage_kernel<T, XM_END, N, E, R0, R1, R2>;
     for (int m : {XM_START, XM_MID, XM_END}) {
-        allow_smem(p.xs[m], (int)p.xbsm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps[m], p.xs[m], p.xw * 32, p.xbsm,
+        allow_smem(p.xs[m], (int)p.xssm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps[m], p.xs[m], p.xw * 32, p.xssm,
                                                               cudaOccupancyDefault);
     }
     for (int m = 0; m < 7; ++m)
