@@ -110,9 +110,12 @@ SES_API ses_status ses_gpu_create_imag(const ses_grid_desc* grid, ses_precision 
 /* relax(Field3D&, nsteps) (imaginary_time.ixx:98-108): nsteps Strang steps of imaginary
  * time, psi renormalised to sum |psi|^2 dV = 1 on the device every renorm_every steps
  * (<= 0: every step, as the reference; the result differs only by rounding since the step
- * is linear).  energy (nullable): -ln(norm^2) / (2 r dtau) over the last r steps before
- * the final renormalisation, which converges to the ground-state energy; with energy
- * NULL the call only queues the work. */
+ * is linear).  Only the first and the last of these renormalisations are certain to be
+ * made: between them up to 33 steps run merged, as far as the range of the precision allows
+ * for this potential, box and dtau, which changes the result by rounding only.  energy
+ * (nullable): -ln(norm^2) / (2 r dtau) over the last r steps before the final
+ * renormalisation, which converges to the ground-state energy; with energy NULL the call
+ * only queues the work. */
 SES_API ses_status ses_gpu_relax(ses_handle h, int nsteps, int renorm_every, double* energy);
 /* Engine::destroy (vk_engine.ixx) */
 SES_API ses_status ses_gpu_destroy(ses_handle h);

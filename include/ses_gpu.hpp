@@ -173,8 +173,8 @@ private:
     ses_handle h_ = nullptr;
 };
 
-// ImaginaryTimePropagator3D (core/src/imaginary_time.ixx:64-108): relax(psi, n)
-// renormalises after every step, as the reference.
+// ImaginaryTimePropagator3D (core/src/imaginary_time.ixx:64-108): relax(psi, n) gives what
+// the reference's renormalisation after every step gives, to rounding (ses_gpu_relax).
 class ImaginaryTimePropagator3D {
 public:
     ImaginaryTimePropagator3D(const Grid3D& g, const std::vector<double>& potential, double dtau,

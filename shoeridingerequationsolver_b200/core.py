@@ -406,7 +406,9 @@ class ImaginaryTimePropagator3D(SplitOperator3D):
     the split-operator step with the real weights exp(-V dtau/2), exp(-k^2 dtau/(2m)),
     renormalised on the device.  ``relax(psi, nsteps)`` keeps the reference's in-place
     semantics on a Field3D; ``relax_resident`` works on the uploaded state and returns
-    the energy estimate -ln(norm^2)/(2 r dtau)."""
+    the energy estimate -ln(norm^2)/(2 r dtau).  ``renorm_every`` sets the first
+    renormalisation, the last one and the r steps of the energy; steps between them run
+    merged as far as the precision's range allows, which changes rounding only."""
 
     def __init__(self, grid: Grid3D, potential, dtau: float, mass: float = 1.0,
                  precision: str = "c128", psi0=None):

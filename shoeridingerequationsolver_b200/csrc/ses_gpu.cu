@@ -991,6 +991,12 @@ ses_status enqueue_renormalize(ses_solver* h) {
 // range e^+-87, transform sums up to N), e^250 in complex128 (the norm is of squares,
 // range e^+-708); at most 33 steps, 4 captured graphs.  64^3 complex128,
 // renormalised after every step: 35 -> 14 us a step.
+//
+// A value of a normalised field is at most dV^-1/2 and one of its transform at most
+// (N / dV)^1/2; the root mean square of the transform / N is (N^2 dV)^-1/2.  Units in
+// which these are far from 1 leave less of the range: the largest value of a growing run
+// stays below e^85 and the root mean square of a shrinking one above e^-68 (complex64 has
+// 7 digits down to e^-87), the sums of squares of complex128 within e^+-700.
 int relax_run(const ses_solver* h) {
     double kmax = 0.0;
     for (int a = 0; a < 3; ++a)
@@ -998,8 +1004,14 @@ int relax_run(const ses_solver* h) {
             const double k = 3.14159265358979323846 * phys_n(h, a) / (h->box[2 * a + 1] - h->box[2 * a]);
             kmax += 0.5 * k * k / h->mass;
         }
-    const double per_step = h->dt * std::max(std::max(h->vmax, 0.0) + kmax, std::max(-h->vmin, 0.0));
-    const double most = (h->prec == SES_C128 ? 250.0 : 48.0) / per_step;
+    double dv = 1.0;
+    for (int a = 0; a < 3; ++a) dv *= (h->box[2 * a + 1] - h->box[2 * a]) / phys_n(h, a);
+    const double top = 0.5 * std::log((double)h->N / dv), rms = -0.5 * std::log((double)h->N * (double)h->N * dv);
+    const bool f64 = h->prec == SES_C128;
+    const double grow = std::min(f64 ? 250.0 : 48.0, (f64 ? 350.0 : 85.0) - top);
+    const double shrink = std::min(f64 ? 250.0 : 48.0, (f64 ? 350.0 : 68.0) + rms);
+    const double most = std::min(grow / (h->dt * std::max(-h->vmin, 0.0)),
+                                 shrink / (h->dt * (std::max(h->vmax, 0.0) + kmax)));
     return most >= 33.0 ? 33 : (most >= 2.0 ? (int)most : 1);  // also 1 when V is not finite
 }
 
