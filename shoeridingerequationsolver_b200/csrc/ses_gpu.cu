@@ -444,7 +444,6 @@ PassArgs<T> make_args(const ses_solver* h, int axis, const void* src, void* dst)
     PassArgs<T> a{};
     a.src = reinterpret_cast<const cx<T>*>(src);
     a.dst = reinterpret_cast<cx<T>*>(dst);
-    a.g = h->pp[axis].g;
     a.axis = axis;
     a.nx = h->n[0];
     a.ny = h->n[1];
@@ -511,8 +510,9 @@ cudaError_t launch_pass(bool pdl, void (*k)(KArgs...), unsigned grid, unsigned b
 
 // A pass on the run-time plan of its axis (steps: of an XM_1D run).
 template <typename T>
-ses_status launch_line(const ses_solver* h, int axis, int mode, PassArgs<T> a, int steps, cudaStream_t s) {
+ses_status launch_line(const ses_solver* h, int axis, int mode, const PassArgs<T>& pass, int steps, cudaStream_t s) {
     const PassPlan& pp = h->pp[axis];
+    LineArgs<T> a{pass, pp.g};
     a.stw = reinterpret_cast<const cx<T>*>(h->ltw[axis]);
     a.stwl = reinterpret_cast<const cx<T>*>(h->ltwl[axis]);
     const unsigned block = (unsigned)pp.g.nthreads;

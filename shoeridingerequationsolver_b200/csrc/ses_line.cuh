@@ -53,6 +53,13 @@ __device__ __forceinline__ void with_radix(int R, F&& f) {
     }
 }
 
+// A pass's arguments and the plan of its axis (kept out of PassArgs, which every other
+// kernel takes too).
+template <typename T>
+struct LineArgs : PassArgs<T> {
+    LinePlan g;
+};
+
 // Contiguous tiles: line l at l * pitch, one spare element after every 16, which
 // spreads the writes of a first stage (R apart) over the banks.
 __host__ __device__ constexpr int line_pad(int pos) { return pos + (pos >> 4); }
@@ -70,15 +77,15 @@ __host__ __device__ constexpr int line_pad(int pos) { return pos + (pos >> 4); }
 // then the two exchange buffers of g.buf.
 template <typename T>
 constexpr size_t line_args_bytes() {
-    return (sizeof(PassArgs<T>) + 15) / 16 * 16;
+    return (sizeof(LineArgs<T>) + 15) / 16 * 16;
 }
 __device__ __forceinline__ unsigned char* line_smem() {
     extern __shared__ __align__(16) unsigned char smraw[];
     return smraw;
 }
 template <typename T>
-__device__ __forceinline__ const PassArgs<T>& line_args() {
-    return *reinterpret_cast<const PassArgs<T>*>(line_smem());
+__device__ __forceinline__ const LineArgs<T>& line_args() {
+    return *reinterpret_cast<const LineArgs<T>*>(line_smem());
 }
 template <typename T>
 __device__ __forceinline__ cx<T>* line_bufs() {
@@ -86,11 +93,11 @@ __device__ __forceinline__ cx<T>* line_bufs() {
 }
 // Copies the arguments in and waits for the previous kernel of the stream.
 template <typename T>
-__device__ __forceinline__ void line_begin(const PassArgs<T>& args) {
-    static_assert(sizeof(PassArgs<T>) % 4 == 0, "copied by words");
+__device__ __forceinline__ void line_begin(const LineArgs<T>& args) {
+    static_assert(sizeof(LineArgs<T>) % 4 == 0, "copied by words");
     const uint32_t* from = reinterpret_cast<const uint32_t*>(&args);
     uint32_t* to = reinterpret_cast<uint32_t*>(line_smem());
-    for (int i = threadIdx.x; i < (int)(sizeof(PassArgs<T>) / 4); i += blockDim.x) to[i] = from[i];
+    for (int i = threadIdx.x; i < (int)(sizeof(LineArgs<T>) / 4); i += blockDim.x) to[i] = from[i];
     pdl_wait();
     __syncthreads();
 }
@@ -106,7 +113,7 @@ template <class P, int R>
 __device__ __forceinline__ void line_stage(P& pass, const LineStage c) {
     using T = typename P::type;
     constexpr bool CONTIG = P::kContig;
-    const PassArgs<T>& a = line_args<T>();
+    const LineArgs<T>& a = line_args<T>();
     const LinePlan& g = a.g;
     cx<T>* bufs = line_bufs<T>();
     const int n = g.n, nR = n / R;
@@ -219,7 +226,7 @@ __device__ __forceinline__ void line_diag_as(const cx<T>* tab, const double* mro
 // The same for line (y, z) = (jy, kz) whose first point is flat index f0, the tests of
 // the pass's program (kind, mask) made once per butterfly.
 template <typename T, bool KICK, int R>
-__device__ __forceinline__ void line_diag(const PassArgs<T>& a, int kind, int msk, long long f0, int j, int nR, int jy,
+__device__ __forceinline__ void line_diag(const LineArgs<T>& a, int kind, int msk, long long f0, int j, int nR, int jy,
                                           int kz, cx<T> (&v)[R]) {
     const Tables& tb = a.tb;
     const cx<T>* tab = reinterpret_cast<const cx<T>*>(tb.vtab) + f0 + j;
@@ -264,7 +271,7 @@ struct LineX {
 
     // coordinates of line l; lines past the end work on line 0
     __device__ __forceinline__ long long line(int l, int* j, int* k) const {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         const long long m = m0 + l < a.nlines ? m0 + l : 0;
         *k = (int)fdiv((uint32_t)m, a.fny);
         *j = (int)(m - (long long)*k * a.ny);
@@ -272,7 +279,7 @@ struct LineX {
     }
     template <int R>
     __device__ __forceinline__ void diag(int kind, int msk, int l, int j, int nR, cx<T> (&v)[R]) const {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         if (kind == DG_NONE && !msk && !KICK) return;
         int jy, kz;
         const long long m = line(l, &jy, &kz);
@@ -285,7 +292,7 @@ struct LineX {
     }
     template <int R>
     __device__ __forceinline__ void load(int l, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         const long long m = m0 + l < a.nlines ? m0 + l : 0;
         const cx<T>* src = a.src + m * a.g.n + j;
 #pragma unroll
@@ -295,7 +302,7 @@ struct LineX {
     }
     template <int R>
     __device__ __forceinline__ void cross(int i, int l, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         if (MODE == XM_MID || (MODE == XM_1D && (i & 1))) {
             conj_all<R>(v);
             diag<R>(a.d_mid, a.m_mid, l, j, nR, v);
@@ -310,7 +317,7 @@ struct LineX {
     }
     template <int R>
     __device__ __forceinline__ void store(int l, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         if constexpr (MODE == XM_REDUCE) {
             if (m0 + l >= a.nlines) return;
             int jy, kz;
@@ -345,9 +352,9 @@ struct LineX {
 // first load to the last store.
 template <typename T, int MODE, int RM, bool KICK>
 __global__ void __launch_bounds__(kLineThreads, (MODE == XM_1D || MODE == XM_REDUCE) ? 1 : line_min_ctas<T, RM>())
-    line_x_kernel(const __grid_constant__ PassArgs<T> args, int steps) {
+    line_x_kernel(const __grid_constant__ LineArgs<T> args, int steps) {
     line_begin(args);
-    const PassArgs<T>& a = line_args<T>();
+    const LineArgs<T>& a = line_args<T>();
     LineX<T, MODE, KICK> pass{(long long)blockIdx.x * a.g.L, {0, 0, 0, 0, 0}};
     line_transforms<RM>(pass, MODE == XM_START, MODE == XM_MID ? 1 : (MODE == XM_1D ? 2 * steps - 1 : 0));
     if constexpr (MODE == XM_REDUCE) block_reduce_store<kRedK>(pass.acc, a.partials);
@@ -366,7 +373,7 @@ struct LineS {
 
     template <int R>
     __device__ __forceinline__ void load(int, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         const cx<T>* src = a.src + base + j * a.se;
         const long long step = nR * a.se;
 #pragma unroll
@@ -378,7 +385,7 @@ struct LineS {
     }
     template <int R>
     __device__ __forceinline__ void cross(int, int, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         if constexpr (MODE == SM_FUSED) {
             const bool ypass = a.axis == 1;
             const cx<double>* kda = ypass ? a.tb.kd[1] : a.tb.kd[2];
@@ -391,7 +398,7 @@ struct LineS {
     }
     template <int R>
     __device__ __forceinline__ void store(int, int j, int nR, cx<T> (&v)[R]) {
-        const PassArgs<T>& a = line_args<T>();
+        const LineArgs<T>& a = line_args<T>();
         if (!valid) return;
         if constexpr (MODE == SM_REDUCE) {
             const bool ypass = a.axis == 1;
@@ -419,9 +426,9 @@ struct LineS {
 
 template <typename T, int MODE, int RM>
 __global__ void __launch_bounds__(kLineThreads, MODE == SM_REDUCE ? 1 : line_min_ctas<T, RM>())
-    line_s_kernel(const __grid_constant__ PassArgs<T> args) {
+    line_s_kernel(const __grid_constant__ LineArgs<T> args) {
     line_begin(args);
-    const PassArgs<T>& a = line_args<T>();
+    const LineArgs<T>& a = line_args<T>();
     const long long s = (long long)blockIdx.x * a.g.L + (threadIdx.x & (a.g.L - 1));
     const bool valid = s < a.nlines;
     const long long sc_ = valid ? s : 0;
@@ -438,9 +445,9 @@ __global__ void __launch_bounds__(kLineThreads, MODE == SM_REDUCE ? 1 : line_min
 }
 
 template <typename T>
-using LineXKernel = void (*)(const PassArgs<T>, int);
+using LineXKernel = void (*)(const LineArgs<T>, int);
 template <typename T>
-using LineSKernel = void (*)(const PassArgs<T>);
+using LineSKernel = void (*)(const LineArgs<T>);
 
 // The kernel of a mode for plans of radices up to rmax (ses_line_c64.cu, ses_line_c128.cu);
 // kick: the modes that apply the potential in driven steps.
