@@ -195,6 +195,12 @@ bool plan_pass(int n, int esize, bool strided, long long nlines, PassPlan& pp, s
     while (L > 1 && smem_of(L) > 200 * 1024) L /= 2;
     while (L > least && (nlines + L - 1) / L < 2 * 148 && L / 2 * widest >= 32) L /= 2;
     while (L > 1 && L / 2 >= nlines) L /= 2;
+    // Fewer tiles than SMs: narrower ones, down to a line, while that puts more SMs to work
+    // or (rows of 32 bytes left) takes a second butterfly off a thread.  us a step, rows of
+    // 64 bytes -> this, complex64: 64 x 1536 33.0 -> 15.5, 256 x 1000 30.2 -> 15.7.
+    while (strided && L > 1 && (nlines + L - 1) / L < 148 && L / 2 * widest >= 32 &&
+           (2 * ((nlines + L - 1) / L) <= 148 || (L * widest > kLineThreads && L / 2 * esize >= 32)))
+        L /= 2;
     LinePlan& g = pp.g;
     g = LinePlan{};
     g.n = n;

@@ -1,0 +1,59 @@
+"""The kernels that a handle's passes run on by default: by axis length, precision and
+the number of lines of the pass, reported by plan_info as they are launched, and the same
+results whichever kernel a pass runs on.
+
+Tolerances between two kernels of one pass and against the FP64 oracle are those of the
+suite: 1e-14 (complex128) / 2e-7 (complex64) and 1e-12 a step / 1e-5 relative L2."""
+
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def plain_environment(monkeypatch, tmp_path):
+    for name in ("SES_XVAR", "SES_SVAR", "SES_PIPELINED", "SES_LONG"):
+        monkeypatch.delenv(name, raising=False)
+    monkeypatch.setenv("SES_TUNE_CACHE", str(tmp_path / "none.txt"))
+    monkeypatch.setenv("SES_PLANE", "0")
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def grid(ses, dims):
+    return ses.Grid3D(*(ses.Grid1D(-7.0, 7.0, d) if d > 1 else ses.Grid1D(0.0, 1.0, 1) for d in dims))
+
+
+def scene(ses, dims, seed=0):
+    rng = np.random.default_rng([seed, *dims])
+    g = grid(ses, dims)
+    return g, rng.uniform(0.0, 3.0, g.size()), rng.standard_normal(g.size()) + 1j * rng.standard_normal(g.size())
+
+
+def parts(op):
+    return dict(zip("xyz", op.plan_info().split("; ")[:3]))
+
+
+# ---- run-time plans with few lines along y or z: tiles of 1, 2 and 4 lines ----
+
+NARROW = [(64, 1536, 1), (5, 1500, 1), (128, 1000, 1), (256, 300, 1), (100, 2048, 1), (256, 4096, 1), (512, 1000, 1),
+          (512, 1536, 1), (20, 1000, 8), (9, 15, 1080), (3, 2, 2000), (1, 27, 750), (250, 1, 600)]
+
+
+@pytest.mark.parametrize("prec", ["c64", "c128"])
+@pytest.mark.parametrize("dims", NARROW, ids=["x".join(map(str, d)) for d in NARROW])
+def test_narrow_tiles(ses, oracle, dims, prec):
+    g, V, psi = scene(ses, dims)
+    op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
+    op.advance(3)
+    assert rel(op.readback(), oracle.step3d(g.box, dims, V, 0.01, psi, 3)) < (3e-12 if prec == "c128" else 1e-5)
+    op.upload_state(psi)
+    op.fft3()
+    want = np.fft.fftn(psi.reshape(g.shape)).reshape(-1)
+    assert rel(op.readback(), want) < (1e-14 if prec == "c128" else 5e-7) * np.log2(g.size())
+    op.close()
