@@ -292,7 +292,8 @@ struct ses_solver {
     bool pdl = true;  // single-field passes launched with programmatic stream serialization
     long long wait_limit = 0;      // failure-detection hook: bounded-wait limit of pipelined passes (0: ~2 s)
     uint32_t extra_tx = 0;         // failure-detection hook: bytes each tile barrier expects beyond its copies
-    int xsel = -1;                 // pipelined contiguous-pass variant (-1: register path, kXStaged: staged rows)
+    int xsel = -1;                 // between-steps contiguous pass (-1: register path, kXStaged: staged rows, else a variant)
+    int xrest = -1;                // pipelined variant of the other contiguous passes (-1: register path); same bits
     int ssel[3] = {-1, -1, -1};    // pipelined strided-pass variant per axis (-1: register path)
     // two-sweep 3D step (plane pass with the y transforms, then the z pass) when
     // the x-y plane fits in shared memory: the compiled plane pass (nullptr: not
@@ -534,59 +535,66 @@ ses_status launch_line(const ses_solver* h, int axis, int mode, const PassArgs<T
     return SES_OK;
 }
 
+// Most lines of a plain transform on the TMA-fed tiles.  Its loads have no kick between
+// them, and beyond this the register path is quicker (TMA-fed / register path, us: transform
+// and inverse of 160^3 complex64 105 / 96, reading of 256^3 complex128 404 / 384).
+constexpr long long kFedForwardLines = 4096;
+
+// The kernel of a contiguous pass: kXStaged, a pipelined variant's index, or -1 (register path).
+template <typename T>
+int x_choice(const ses_solver* h, int mode) {
+    const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[0].cp);
+    if (!e || !h->pipelined || (mode == XM_FWD && h->pp[0].nlines > kFedForwardLines)) return -1;
+    const int v = mode == XM_MID ? h->xsel : h->xrest;
+    if (v == kXStaged) return e->xs_bps > 0 ? kXStaged : -1;
+    return v >= 0 && v < (int)e->xv.size() && e->xv[v].k[mode] && e->xv[v].bps[mode] > 0 ? v : -1;
+}
+
+// The kernel of an in-place strided pass on psi (buf 0) or scratch (1): a pipelined variant's index, or -1.
+template <typename T>
+int s_choice(const ses_solver* h, int axis, int mode, int buf) {
+    const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[axis].cp);
+    const int v = h->ssel[axis];
+    if (!e || !h->pipelined || v < 0 || v >= (int)e->sv.size() || v >= ses_solver::kMaxVar) return -1;
+    return e->sv[v].k[mode] && e->sv[v].bps[mode] > 0 && h->tmap_ok[buf][axis][v] &&
+                   (axis == 2 || h->n[0] % e->sv[v].ls == 0) ? v : -1;
+}
+
 template <typename T>
 ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a, cudaStream_t s) {
     const PassPlan& pp = h->pp[axis];
     if (!pp.cp) return launch_line<T>(h, axis, mode, a, 1, s);
-    {
-        const PlanEntry<T>* e = reinterpret_cast<const PlanEntry<T>*>(pp.cp);
-        const int n = h->n[axis];
-        bool done = false;
-        const int xs = h->xsel, ss = h->ssel[axis];
-        if (h->pipelined && axis == 0 && xs == kXStaged && e->xs[mode] && e->xs_bps[mode] > 0) {
-            const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps[mode]));
-            launch_pass(h->pdl, e->xs[mode], grid, pp.cblock, e->xssm, s, a, (uint32_t)pp.cgrid);
-            done = true;
-        } else if (h->pipelined && axis == 0 && xs >= 0 && xs < (int)e->xv.size() && e->xv[xs].k[mode] &&
-            e->xv[xs].bps[mode] > 0) {
-            const auto& v = e->xv[xs];
-            PipeArgs pa{};
-            pa.ntiles = (int)((pp.nlines + v.lpc - 1) / v.lpc);
-            pa.err = h->herr;
-            pa.wait_limit = h->wait_limit;
-            pa.extra_tx = h->extra_tx;
-            const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
-            launch_pass(h->pdl, v.k[mode], (unsigned)grid, 32u * v.warps, v.smem[mode], s, a, pa);
-            done = true;
-        } else if (h->pipelined && axis != 0 && ss >= 0 && ss < (int)e->sv.size() && e->sv[ss].k[mode] &&
-                   e->sv[ss].bps[mode] > 0) {
-            const auto& v = e->sv[ss];
-            const int buf = a.src == reinterpret_cast<const cx<T>*>(h->psi) ? 0
-                            : (a.src == reinterpret_cast<const cx<T>*>(h->scratch) ? 1 : -1);
-            if (buf >= 0 && ss < ses_solver::kMaxVar && h->tmap_ok[buf][axis][ss] && a.src == a.dst &&
-                (axis == 2 || h->n[0] % v.ls == 0)) {
-                PipeArgs pa{};
-                pa.ntiles = (int)((pp.nlines + v.ls - 1) / v.ls);
-                pa.kind = axis == 1 ? 0 : 1;
-                pa.rows_per_box = n > 256 ? 256 : n;
-                pa.nbox = n / pa.rows_per_box;
-                pa.err = h->herr;
-                pa.wait_limit = h->wait_limit;
-                pa.extra_tx = h->extra_tx;
-                const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
-                launch_pass(h->pdl, v.k[mode], (unsigned)grid, (unsigned)v.threads, v.smem, s, a,
-                            h->tmap[buf][axis][ss], pa);
-                done = true;
-            }
-        }
-        if (!done) {
-            PassKernel<T> k = axis == 0 ? e->xk[mode] : e->sk[mode];
-            launch_pass(h->pdl, k, pp.cgrid, pp.cblock, pp.csmem, s, a);
-        }
+    const PlanEntry<T>* e = reinterpret_cast<const PlanEntry<T>*>(pp.cp);
+    const int n = h->n[axis];
+    const int buf = a.src == reinterpret_cast<const cx<T>*>(h->psi) ? 0
+                    : (a.src == reinterpret_cast<const cx<T>*>(h->scratch) ? 1 : -1);
+    const int var = axis == 0 ? x_choice<T>(h, mode)
+                              : (buf >= 0 && a.src == a.dst ? s_choice<T>(h, axis, mode, buf) : -1);
+    PipeArgs pa{};
+    pa.err = h->herr;
+    pa.wait_limit = h->wait_limit;
+    pa.extra_tx = h->extra_tx;
+    if (var < 0) {
+        launch_pass(h->pdl, axis == 0 ? e->xk[mode] : e->sk[mode], pp.cgrid, pp.cblock, pp.csmem, s, a);
+    } else if (axis == 0 && var == kXStaged) {
+        const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps));
+        launch_pass(h->pdl, e->xs, grid, pp.cblock, e->xssm, s, a, (uint32_t)pp.cgrid);
+    } else if (axis == 0) {
+        const auto& v = e->xv[var];
+        pa.ntiles = (int)((pp.nlines + v.lpc - 1) / v.lpc);
+        const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
+        launch_pass(h->pdl, v.k[mode], (unsigned)grid, 32u * v.warps, v.smem[mode], s, a, pa);
+    } else {
+        const auto& v = e->sv[var];
+        pa.ntiles = (int)((pp.nlines + v.ls - 1) / v.ls);
+        pa.kind = axis == 1 ? 0 : 1;
+        pa.rows_per_box = n > 256 ? 256 : n;
+        pa.nbox = n / pa.rows_per_box;
+        const int grid = std::min(pa.ntiles, h->sms * v.bps[mode]);
+        launch_pass(h->pdl, v.k[mode], (unsigned)grid, (unsigned)v.threads, v.smem, s, a, h->tmap[buf][axis][var], pa);
     }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess)
-        return fail(SES_EDEVICE, std::string("pass launch: ") + cudaGetErrorString(e));
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return fail(SES_EDEVICE, std::string("pass launch: ") + cudaGetErrorString(err));
     return SES_OK;
 }
 
@@ -1321,9 +1329,19 @@ void default_variants(ses_solver* h) {
     for (int a = 0; a < 3; ++a) {
         const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[a].cp);
         if (!e) continue;
-        if (a == 0) h->xsel = e->xdef;
-        else h->ssel[a] = a == h->last_axis ? e->fdef : e->sdef;
+        if (a == 0) {
+            h->xsel = e->xdef;
+            h->xrest = h->pp[a].nlines <= e->xrest_lines ? e->xrest : -1;
+        } else h->ssel[a] = a == h->last_axis ? e->fdef : e->sdef;
     }
+}
+
+// A given selection of the between-steps contiguous pass.  A pipelined variant serves the
+// other contiguous passes too; staged rows and the register path leave them theirs.
+// (Steps of a line make none between them: there a selection is that of the others.)
+void select_x(ses_solver* h, int v) {
+    h->xsel = v;
+    if (v != kXStaged && (v >= 0 || h->last_axis == 0)) h->xrest = v;
 }
 
 // Selections at creation: defaults, cache, then environment overrides SES_XVAR / SES_SVAR / SES_PLANE.
@@ -1335,7 +1353,7 @@ void apply_selection(ses_solver* h) {
     for (int a = 0; a < 3; ++a) {
         auto it = cache.find(tune_key(h, a));
         if (it == cache.end()) continue;
-        if (a == 0) h->xsel = it->second;
+        if (a == 0) select_x(h, it->second);
         else h->ssel[a] = it->second;
     }
     if (has_planes(h)) {  // cached choice, then SES_PLANE (CTAs per plane; 0 = four axis passes)
@@ -1343,7 +1361,10 @@ void apply_selection(ses_solver* h) {
         if (it != cache.end()) apply_plane_choice(h, it->second);
         if (const char* e = std::getenv("SES_PLANE")) apply_plane_choice(h, std::atoi(e));
     }
-    if (const char* e = std::getenv("SES_XVAR")) h->xsel = std::atoi(e);
+    if (const char* e = std::getenv("SES_XVAR")) {
+        select_x(h, std::atoi(e));
+        if (h->xsel < 0) h->xrest = -1;  // the register path in every pass
+    }
     if (const char* e = std::getenv("SES_PDL")) h->pdl = std::atoi(e) != 0;
     if (const char* e = std::getenv("SES_SVAR")) h->ssel[1] = h->ssel[2] = std::atoi(e);
 }
@@ -1424,11 +1445,12 @@ ses_status autotune_impl(ses_solver* h, int flags) {
         const int nv = variant_count<T>(h, axis);
         int best = -1;
         float best_ms = 1e30f;
+        const int rest = h->xrest;
         std::vector<int> variants;
         for (int c = -1; c < nv; ++c) variants.push_back(c);
         if (axis == 0 && h->last_axis > 0) variants.push_back(kXStaged);
         for (int c : variants) {
-            if (axis == 0) h->xsel = c;
+            if (axis == 0) select_x(h, c);
             else h->ssel[axis] = c;
             float ms = 0.f;
             SES_TRY(time_axis_pass<T>(h, axis, 5, &ms));
@@ -1437,7 +1459,8 @@ ses_status autotune_impl(ses_solver* h, int flags) {
                 best = c;
             }
         }
-        if (axis == 0) h->xsel = best;
+        h->xrest = rest;
+        if (axis == 0) select_x(h, best);
         else h->ssel[axis] = best;
         chosen[tune_key(h, axis)] = best;
     }
@@ -1496,6 +1519,8 @@ std::string plan_info_t(const ses_solver* h) {
                 o << (e->sv[sel].swizzle ? " pipelined TMA warp lines=" : " pipelined TMA lines=") << e->sv[sel].ls << " ring=" << e->sv[sel].nbuf << " (variant "
                   << sel << ")";
             }
+            const int ends = a == 0 && h->last_axis > 0 && !h->long1d ? x_choice<T>(h, XM_START) : sel;
+            if (ends != sel) o << (ends < 0 ? ", ends register-path" : ", ends pipelined");
         }
         if (a < 2) o << "; ";
     }
@@ -1970,7 +1995,7 @@ struct BatchClass {
     void* dargs = nullptr; // [prog][mask][member] PassArgs<T>
     size_t dcap = 0;
     // pipelined (TMA-fed) batched variants: -1 = register-path batched kernels
-    int xvar = -1;
+    int xvar = -1, xrest = -1;  // x pass between steps; first and last x pass of a call
     int svar[3] = {-1, -1, -1};
     CUtensorMap* dmaps = nullptr;  // [strided pass q][member] tensor maps of the members' psi
     size_t mcap = 0;
@@ -2131,7 +2156,7 @@ bool svar_ok(const BatchClass& c, int q, int k, int buf) {
 template <typename T>
 void class_select(const ses_batch_s* b, BatchClass& c) {
     const ses_solver* h0 = c.mem[0];
-    c.xvar = -1;
+    c.xvar = c.xrest = -1;
     for (int q = 0; q < 3; ++q) c.svar[q] = -1;
     if (!h0->pipelined || h0->last_axis == 0) return;
     const std::map<std::string, int> cache = read_tune_cache();
@@ -2143,8 +2168,11 @@ void class_select(const ses_batch_s* b, BatchClass& c) {
         if (jt != cache.end()) return jt->second;
         return fallback;
     };
-    const int xs = pick(0, -1);  // the staged rows of the register path were fastest for every length
-    if (xvar_ok<T>(c, xs)) c.xvar = xs;
+    // by default the staged rows of the register path, the fastest for every length between steps
+    const int xs = pick(0, -1);
+    const int rest = reinterpret_cast<const PlanEntry<T>*>(h0->pp[0].cp)->xrest;
+    if (xvar_ok<T>(c, xs)) c.xvar = c.xrest = xs;
+    else if (xvar_ok<T>(c, rest)) c.xrest = rest;
     for (int q = 0; q < c.nmid; ++q) {
         const auto* e = reinterpret_cast<const PlanEntry<T>*>(h0->pp[c.mid_axis[q]].cp);
         const int ss = pick(1 + q, !e ? -1 : (c.mid_mode[q] == SM_FUSED ? e->bfdef : e->bsdef));
@@ -2396,14 +2424,14 @@ ses_status class_launch(const ses_batch_s* b, const BatchClass& c, int prog, boo
         args_ovr ? args_ovr : reinterpret_cast<const PassArgs<T>*>(c.dargs) + ((size_t)prog * 2 + (mask ? 1 : 0)) * nm;
     const CUtensorMap* maps = maps_ovr ? maps_ovr : c.dmaps;
     const int q = prog - BP_MID0;
-    if (prog < BP_LSTART && (axis == 0 ? c.xvar >= 0 && (mode == XM_START || mode == XM_MID || mode == XM_END)
-                                       : c.svar[q] >= 0)) {
+    const int xvar = mode == XM_MID ? c.xvar : (mode == XM_START || mode == XM_END ? c.xrest : -1);
+    if (prog < BP_LSTART && (axis == 0 ? xvar : c.svar[q]) >= 0) {
         const int n = h0->n[axis];
         PipeArgs pa{};
         pa.err = b->herr;
         BatchWork w{};
         if (axis == 0) {
-            const auto& v = e->xv[c.xvar];
+            const auto& v = e->xv[xvar];
             w.bpi = (uint32_t)((pp.nlines + v.lpc - 1) / v.lpc);
         } else {
             const auto& v = e->sv[c.svar[q]];
@@ -2418,7 +2446,7 @@ ses_status class_launch(const ses_batch_s* b, const BatchClass& c, int prog, boo
         w.fbpi = make_fastdiv(w.bpi);
         pa.ntiles = (int)w.total;
         if (axis == 0) {
-            const auto& v = e->xv[c.xvar];
+            const auto& v = e->xv[xvar];
             const unsigned grid = std::min<unsigned>(w.total, (unsigned)(b->sms * v.bbps[mode]));
             launch_pass(h0->pdl, v.kb[mode], grid, 32u * v.warps, v.smemb[mode], s, args, w, pa);
         } else {

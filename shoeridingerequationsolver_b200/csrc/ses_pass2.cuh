@@ -650,15 +650,14 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     }
 }
 
-// The same for one field (mode START, MID or END): CTAs walk its line tiles with the
-// stage twiddles in shared memory and each tile's potential rows and absorber profile
-// fetched by cp.async while its first transform runs.  Bound by issue and latency (80 us
-// for the 403 MB of a 256^3 complex64 pass, whose copy takes 61).  Between steps, n^3
-// fields, us, TMA-fed or register path -> staged rows: complex64 128 18.7 -> 16.5, 256
-// 93.1 -> 80.6, 512 857 -> 678; complex128 64 9.6 -> 8.3, 128 27.8 -> 22.6, 256 159 -> 132.
-// The absorber's x profile is one field's, so a CTA stages it once: with a copy per warp
-// and tile it took a third of the staged bytes and, at 512 points, a CTA of the SM
-// (512^3 pass 709 -> 678 us; 1024^2 step 28.0 -> 22.6).
+// The between-steps pass of one field: CTAs walk its line tiles with the stage twiddles
+// in shared memory and each tile's potential rows fetched by cp.async while its first
+// transform runs.  Bound by issue and latency (80 us for the 403 MB of a 256^3 complex64
+// pass, whose copy takes 61).  n^3 fields, us, TMA-fed or register path -> staged rows:
+// complex64 128 18.7 -> 16.5, 256 93.1 -> 80.6, 512 857 -> 678; complex128 64 9.6 -> 8.3,
+// 128 27.8 -> 22.6, 256 159 -> 132.  The absorber's x profile is one field's, so a CTA
+// stages it once: with a copy per warp and tile it took a third of the staged bytes and,
+// at 512 points, a CTA of the SM (512^3 pass 709 -> 678 us; 1024^2 step 28.0 -> 22.6).
 template <typename T, int N, int E, int R0, int R1, int R2>
 constexpr size_t xstage_smem() {
     return TwStage<T, R0, R1, R2>::bytes +
@@ -666,7 +665,7 @@ constexpr size_t xstage_smem() {
            (size_t)N * sizeof(double);
 }
 
-template <typename T, int MODE, int N, int E, int R0, int R1, int R2>
+template <typename T, int N, int E, int R0, int R1, int R2>
 __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MINB)
     xstage_kernel(const __grid_constant__ PassArgs<T> a, const uint32_t tiles) {
     using XS = XShape<T, N, E>;
@@ -681,20 +680,15 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     if (a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr)
         for (int i = threadIdx.x; i < N; i += blockDim.x) mrow[i] = a.tb.mask1[0][i];
     __syncthreads();
-    const int form = MODE == XM_MID ? kick_form(a) : (int)KICK_ANY;
+    const int form = kick_form(a);
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const long long tile = (long long)t;
-        if constexpr (MODE == XM_MID) {
-            if (form == KICK_SEP) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
-                continue;
-            }
-            if (form == KICK_PLAIN) {
-                xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_PLAIN, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
-                continue;
-            }
-        }
-        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
+        if (form == KICK_SEP)
+            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_SEP, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
+        else if (form == KICK_PLAIN)
+            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_PLAIN, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
+        else
+            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_ANY, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
     }
 }
 

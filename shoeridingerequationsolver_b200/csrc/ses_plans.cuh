@@ -1,6 +1,6 @@
 // Registry of compiled line-FFT plans (axis length -> radices, elements per
 // thread, strided-pass tile width) and their kernels.  Lengths without an
-// entry run on the run-time-plan kernels of ses_pass.cuh.
+// entry run on the run-time-plan kernels of ses_line.cuh.
 #pragma once
 
 #include <vector>
@@ -14,7 +14,7 @@ namespace sesk {
 template <typename T>
 using PassKernel = void (*)(const PassArgs<T>);
 
-constexpr int kXStaged = 64;  // contiguous-pass selection: the staged-rows kernel
+constexpr int kXStaged = 64;  // contiguous-pass selection: staged rows between steps
 
 template <typename T>
 struct PlanEntry {
@@ -26,7 +26,7 @@ struct PlanEntry {
     size_t xbsm = 0;        // dynamic shared memory of the batched register-path x pass
     PassKernel<T> xk[7];    // by XMode
     PassKernel<T> sk[kSModes];  // by SModeK
-    // pipelined variants; the solver picks one per axis (default 0, or autotuned)
+    // pipelined variants; the solver picks one per axis (the plan's default, or autotuned)
     using XPipe = void (*)(const PassArgs<T>, const PipeArgs);
     using SPipe = void (*)(const PassArgs<T>, const CUtensorMap, const PipeArgs);
     // batched forms: per-instance arguments (and tensor maps) in global memory
@@ -53,15 +53,17 @@ struct PlanEntry {
     };
     std::vector<XVar> xv;
     std::vector<SVar> sv;
-    // contiguous passes of one field on staged rows (xstage_kernel), by XMode
+    // the between-steps contiguous pass of one field on staged rows (xstage_kernel)
     using XStage = void (*)(const PassArgs<T>, uint32_t);
-    XStage xs[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int xs_bps[7] = {0, 0, 0, 0, 0, 0, 0};
+    XStage xs = nullptr;
+    int xs_bps = 0;
     size_t xssm = 0;
     // default variants (a pipelined variant's index, -1 the register path, x: kXStaged),
-    // as measured: contiguous passes, strided passes, strided passes with the kinetic
-    // phase, and the strided ones of batches
-    int xdef = kXStaged, sdef = -1, fdef = -1, bsdef = -1, bfdef = -1;
+    // as measured: the contiguous pass between steps, the other contiguous passes (first
+    // and last of a call, plain transforms of few lines), strided passes, strided passes with the
+    // kinetic phase, and the strided ones of batches
+    int xdef = kXStaged, xrest = -1, sdef = -1, fdef = -1, bsdef = -1, bfdef = -1;
+    long long xrest_lines = 1LL << 62;  // xrest serves passes of at most so many lines
     // batched kernels (many fields of this length per launch), by mode
     using XBatch = void (*)(const PassArgs<T>*, const BatchWork);
     XBatch xb[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -114,14 +116,9 @@ PlanEntry<T> make_plan_entry() {
     p.sb[SM_TW_MID] = sbatch_kernel<T, SM_TW_MID, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_END] = sbatch_kernel<T, SM_TW_END, N, E, R0, R1, R2, LS>;
     p.xssm = xstage_smem<T, N, E, R0, R1, R2>();
-    p.xs[XM_START] = xstage_kernel<T, XM_START, N, E, R0, R1, R2>;
-    p.xs[XM_MID] = xstage_kernel<T, XM_MID, N, E, R0, R1, R2>;
-    p.xs[XM_END] = xstage_kernel<T, XM_END, N, E, R0, R1, R2>;
-    for (int m : {XM_START, XM_MID, XM_END}) {
-        allow_smem(p.xs[m], (int)p.xssm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps[m], p.xs[m], p.xw * 32, p.xssm,
-                                                              cudaOccupancyDefault);
-    }
+    p.xs = xstage_kernel<T, N, E, R0, R1, R2>;
+    allow_smem(p.xs, (int)p.xssm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps, p.xs, p.xw * 32, p.xssm, cudaOccupancyDefault);
     for (int m = 0; m < 7; ++m)
         if (p.xb[m]) {
             allow_smem(p.xb[m], (int)p.xbsm);
@@ -174,6 +171,10 @@ void add_x_variant(PlanEntry<T>& p) {
         }
     }
     cudaGetLastError();
+    // The passes that apply a kick while they load or store and the plain transform: fed by
+    // TMA wherever it is built, us a step of a one-step call, register path or staged rows
+    // -> variant 0: complex64 256 x 256 31 -> 25, 256^3 539 -> 385; complex128 31 -> 25, 1078 -> 822.
+    p.xrest = 0;
     p.xv.push_back(v);
 }
 
@@ -243,6 +244,13 @@ void set_defaults(PlanEntry<T>& p, int x, int s, int f, int bs, int bf) {
     p.fdef = f;
     p.bsdef = bs;
     p.bfdef = bf;
+}
+
+// The other contiguous passes, of at most `lines` lines (more: the register path).
+template <typename T>
+void set_rest(PlanEntry<T>& p, int x, long long lines) {
+    p.xrest = x;
+    p.xrest_lines = lines;
 }
 
 // defined in ses_plans_*.cu

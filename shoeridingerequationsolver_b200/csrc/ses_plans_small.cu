@@ -11,6 +11,7 @@ void register_plans_small(std::vector<PlanEntry<float>>& f, std::vector<PlanEntr
     add_s_variant<float, 32, 8, 8, 4, 1, 32, 2, 4>(f.back());
     add_s_variant<float, 32, 8, 8, 4, 1, 32, 3, 3>(f.back());
     set_defaults(f.back(), kXStaged, 0, 0, 0, 0);
+    set_rest(f.back(), -1, 0);
     d.push_back(make_plan_entry<double, 32, 8, 8, 4, 1, 16>());
     f.push_back(make_plan_entry<float, 64, 8, 8, 8, 1, 32>());
     add_x_variant<float, 64, 8, 8, 8, 1, 4, 2, 2>(f.back());

@@ -39,6 +39,39 @@ def parts(op):
     return dict(zip("xyz", op.plan_info().split("; ")[:3]))
 
 
+# ---- first and last x passes of a call ----
+
+X_VARIANTS = [(32, "c64", False), (48, "c64", False), (64, "c64", True), (96, "c64", True), (128, "c64", True),
+              (160, "c64", True), (256, "c64", True), (512, "c64", True), (1024, "c64", False), (32, "c128", False),
+              (64, "c128", True), (96, "c128", False), (128, "c128", False), (256, "c128", True), (512, "c128", True)]
+
+
+@pytest.mark.parametrize("nx,prec,fed", X_VARIANTS)
+def test_first_and_last_x_passes(ses, nx, prec, fed):
+    """They run on the TMA-fed kernel where one is built (a one-step call of 256^3 complex64
+    takes 385 us so, 539 without), and a run split into calls gives the bits of one call."""
+    dims = (nx, 32, 25 if nx < 512 else 9)
+    g, V, psi = scene(ses, dims)
+    op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
+    x = parts(op)["x"]
+    assert ("pipelined" in x) == fed, x
+    profiles = [np.linspace(0.97, 1.0, d) for d in dims]
+    full = np.random.default_rng(1).uniform(0.97, 1.0, g.size())
+    for mask in (None, "separable", "full"):
+        if mask == "separable":
+            op.set_absorber_separable(*profiles)
+        elif mask == "full":
+            op.set_absorber(full)
+        outs = []
+        for split in ((6,), (1, 1, 1, 1, 1, 1), (2, 4)):
+            op.upload_state(psi)
+            for k in split:
+                op.advance(k, absorb=mask is not None)
+            outs.append(op.readback())
+        assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2]), mask
+    op.close()
+
+
 # ---- run-time plans with few lines along y or z: tiles of 1, 2 and 4 lines ----
 
 NARROW = [(64, 1536, 1), (5, 1500, 1), (128, 1000, 1), (256, 300, 1), (100, 2048, 1), (256, 4096, 1), (512, 1000, 1),
