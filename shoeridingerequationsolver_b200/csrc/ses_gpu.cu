@@ -1329,10 +1329,15 @@ void default_variants(ses_solver* h) {
     for (int a = 0; a < 3; ++a) {
         const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[a].cp);
         if (!e) continue;
+        const long long lines = h->pp[a].nlines;
         if (a == 0) {
-            h->xsel = e->xdef;
-            h->xrest = h->pp[a].nlines <= e->xrest_lines ? e->xrest : -1;
-        } else h->ssel[a] = a == h->last_axis ? e->fdef : e->sdef;
+            h->xsel = lines <= e->xfew_lines ? e->xfew : e->xdef;
+            h->xrest = lines <= e->xrest_lines ? e->xrest : -1;
+        } else if (lines <= e->few_lines) {
+            h->ssel[a] = a == h->last_axis ? e->ffew : e->sfew;
+        } else {
+            h->ssel[a] = a == h->last_axis ? e->fdef : e->sdef;
+        }
     }
 }
 

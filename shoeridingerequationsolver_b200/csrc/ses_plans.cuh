@@ -63,7 +63,10 @@ struct PlanEntry {
     // and last of a call, plain transforms of few lines), strided passes, strided passes with the
     // kinetic phase, and the strided ones of batches
     int xdef = kXStaged, xrest = -1, sdef = -1, fdef = -1, bsdef = -1, bfdef = -1;
+    // the same for passes of at most so many lines: a tile or two per SM, whose latency counts
+    long long xfew_lines = 0, few_lines = 0;
     long long xrest_lines = 1LL << 62;  // xrest serves passes of at most so many lines
+    int xfew = -1, sfew = -1, ffew = -1;
     // batched kernels (many fields of this length per launch), by mode
     using XBatch = void (*)(const PassArgs<T>*, const BatchWork);
     XBatch xb[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -246,11 +249,26 @@ void set_defaults(PlanEntry<T>& p, int x, int s, int f, int bs, int bf) {
     p.bfdef = bf;
 }
 
+// The strided and fused defaults of passes of at most `lines` lines.
+template <typename T>
+void set_few(PlanEntry<T>& p, long long lines, int s, int f) {
+    p.few_lines = lines;
+    p.sfew = s;
+    p.ffew = f;
+}
+
 // The other contiguous passes, of at most `lines` lines (more: the register path).
 template <typename T>
 void set_rest(PlanEntry<T>& p, int x, long long lines) {
     p.xrest = x;
     p.xrest_lines = lines;
+}
+
+// The contiguous default between steps of passes of at most `lines` lines.
+template <typename T>
+void set_few_x(PlanEntry<T>& p, long long lines, int x) {
+    p.xfew_lines = lines;
+    p.xfew = x;
 }
 
 // defined in ses_plans_*.cu

@@ -15,6 +15,7 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<float, 256, 16, 16, 16, 1, 8, 2, 4>(f.back());
     add_s4_variant<float, 256, 16, 16, 16, 64, 4, 12>(f.back());
     set_defaults(f.back(), kXStaged, 4, 4, 4, 4);
+    set_few(f.back(), 4096, 3, 3);
     d.push_back(make_plan_entry<double, 256, 16, 16, 16, 1, 16>());
     add_x_variant<double, 256, 16, 16, 16, 1, 2, 2, 1>(d.back());
     add_x_variant<double, 256, 16, 16, 16, 1, 4, 2, 2>(d.back());
@@ -24,5 +25,7 @@ void register_plans_256(std::vector<PlanEntry<float>>& f, std::vector<PlanEntry<
     add_s_variant<double, 256, 16, 16, 16, 1, 4, 2, 4>(d.back());
     add_s4_variant<double, 256, 16, 16, 16, 64, 6, 12>(d.back());
     set_defaults(d.back(), kXStaged, 3, 3, 3, 3);
+    set_few(d.back(), 2048, 2, 2);
+    set_few_x(d.back(), 512, 0);
 }
 }  // namespace sesk

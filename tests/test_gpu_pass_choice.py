@@ -72,6 +72,40 @@ def test_first_and_last_x_passes(ses, nx, prec, fed):
     op.close()
 
 
+# ---- defaults by the number of lines ----
+
+# (axis, dims with few lines, dims with more, precision, text of the first, text of the second)
+BY_LINES = [("y", (64, 512, 1), (64, 512, 40), "c64", "register-path", "TMA lines=8"),
+            ("z", (16, 128, 512), (32, 72, 512), "c64", "register-path", "warp lines=8"),
+            ("z", (64, 64, 256), (64, 72, 256), "c64", "TMA lines=8", "warp lines=8"),
+            ("y", (64, 256, 64), (64, 256, 65 + 7), "c64", "TMA lines=8", "warp lines=8"),
+            ("z", (64, 128, 128), (96, 96, 128), "c64", "TMA lines=8", "warp lines=16"),
+            ("z", (64, 128, 128), (96, 96, 128), "c128", "register-path", "warp lines=8"),
+            ("y", (128, 128, 64), (128, 128, 72), "c128", "register-path", "warp lines=8"),
+            ("y", (256, 256, 1), (64, 256, 36), "c128", "TMA lines=4", "warp lines=4"),
+            ("z", (32, 64, 256), (36, 64, 256), "c128", "TMA lines=4", "warp lines=4"),
+            ("x", (256, 512, 1), (256, 540, 1), "c128", "pipelined warps=2", "staged rows"),
+            ("x", (512, 256, 1), (512, 270, 1), "c128", "pipelined warps=2", "staged rows")]
+
+
+@pytest.mark.parametrize("axis,few,more,prec,t_few,t_more", BY_LINES)
+def test_defaults_follow_the_number_of_lines(ses, axis, few, more, prec, t_few, t_more):
+    for dims, text in ((few, t_few), (more, t_more)):
+        g, V, psi = scene(ses, dims)
+        op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
+        assert text in parts(op)[axis], (dims, op.plan_info())
+        op.advance(3)
+        got = op.readback()
+        op.close()
+        os.environ["SES_XVAR"] = os.environ["SES_SVAR"] = "-1"
+        op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
+        del os.environ["SES_XVAR"], os.environ["SES_SVAR"]
+        assert "pipelined" not in op.plan_info() and "staged" not in op.plan_info()
+        op.advance(3)
+        assert rel(got, op.readback()) < (1e-14 if prec == "c128" else 2e-7), dims
+        op.close()
+
+
 # ---- run-time plans with few lines along y or z: tiles of 1, 2 and 4 lines ----
 
 NARROW = [(64, 1536, 1), (5, 1500, 1), (128, 1000, 1), (256, 300, 1), (100, 2048, 1), (256, 4096, 1), (512, 1000, 1),
