@@ -546,7 +546,7 @@ int x_choice(const ses_solver* h, int mode) {
     const auto* e = reinterpret_cast<const PlanEntry<T>*>(h->pp[0].cp);
     if (!e || !h->pipelined || (mode == XM_FWD && h->pp[0].nlines > kFedForwardLines)) return -1;
     const int v = mode == XM_MID ? h->xsel : h->xrest;
-    if (v == kXStaged) return e->xs_bps > 0 ? kXStaged : -1;
+    if (v == kXStaged) return std::min({e->xs_bps[0], e->xs_bps[1], e->xs_bps[2]}) > 0 ? kXStaged : -1;
     return v >= 0 && v < (int)e->xv.size() && e->xv[v].k[mode] && e->xv[v].bps[mode] > 0 ? v : -1;
 }
 
@@ -577,8 +577,9 @@ ses_status launch(const ses_solver* h, int axis, int mode, const PassArgs<T>& a,
     if (var < 0) {
         launch_pass(h->pdl, axis == 0 ? e->xk[mode] : e->sk[mode], pp.cgrid, pp.cblock, pp.csmem, s, a);
     } else if (axis == 0 && var == kXStaged) {
-        const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps));
-        launch_pass(h->pdl, e->xs, grid, pp.cblock, e->xssm, s, a, (uint32_t)pp.cgrid);
+        const int form = kick_form(a);
+        const unsigned grid = std::min(pp.cgrid, (unsigned)(h->sms * e->xs_bps[form]));
+        launch_pass(h->pdl, e->xs[form], grid, pp.cblock, e->xssm, s, a, (uint32_t)pp.cgrid);
     } else if (axis == 0) {
         const auto& v = e->xv[var];
         pa.ntiles = (int)((pp.nlines + v.lpc - 1) / v.lpc);
@@ -2002,6 +2003,7 @@ struct BatchClass {
     // pipelined (TMA-fed) batched variants: -1 = register-path batched kernels
     int xvar = -1, xrest = -1;  // x pass between steps; first and last x pass of a call
     int svar[3] = {-1, -1, -1};
+    int form[2] = {KICK_ANY, KICK_ANY};  // KickForm of every member's pass between steps, without and with the absorber
     CUtensorMap* dmaps = nullptr;  // [strided pass q][member] tensor maps of the members' psi
     size_t mcap = 0;
     cudaStream_t cs = nullptr, cap = nullptr;
@@ -2318,6 +2320,12 @@ ses_status class_upload(const ses_batch_s* b, BatchClass& c) {
                 }
                 share_tables(c, i, a);
             }
+    for (int mask = 0; mask < 2; ++mask) {
+        const PassArgs<T>* mid = &host[((size_t)BP_XMID * 2 + mask) * nm];
+        c.form[mask] = kick_form(mid[0]);
+        for (size_t i = 1; i < nm; ++i)
+            if (kick_form(mid[i]) != c.form[mask]) c.form[mask] = KICK_ANY;
+    }
     class_select<T>(b, c);
     c.plane = class_plane<T>(b, c);
     // tensor maps [q][member] of the members' psi for the selected strided variants
@@ -2472,9 +2480,10 @@ ses_status class_launch(const ses_batch_s* b, const BatchClass& c, int prog, boo
     w.total = (uint32_t)(pp.cgrid * nm);
     w.fbpi = make_fastdiv(w.bpi);
     if (axis == 0) {
-        const int bps = std::max(1, e->xb_bps[mode]);
+        const int form = c.form[mask ? 1 : 0];
+        const int bps = std::max(1, mode == XM_MID ? e->xbf_bps[form] : e->xb_bps[mode]);
         const unsigned grid = std::min<unsigned>(w.total, (unsigned)(b->sms * bps));
-        launch_pass(h0->pdl, e->xb[mode], grid, pp.cblock, e->xbsm, s, args, w);
+        launch_pass(h0->pdl, mode == XM_MID ? e->xbf[form] : e->xb[mode], grid, pp.cblock, e->xbsm, s, args, w);
     } else {
         const int bps = std::max(1, e->sb_bps[mode]);
         const unsigned grid = std::min<unsigned>(w.total, (unsigned)(b->sms * bps));

@@ -226,7 +226,7 @@ struct XShape {
 enum KickForm : int { KICK_ANY = 0, KICK_SEP = 1, KICK_PLAIN = 2 };
 
 template <typename T>
-__device__ __forceinline__ int kick_form(const PassArgs<T>& a) {  // of a between-steps pass
+__host__ __device__ __forceinline__ int kick_form(const PassArgs<T>& a) {  // of a between-steps pass
     if (a.d_mid != DG_FULL) return KICK_ANY;
     if (!a.m_mid) return KICK_PLAIN;
     return a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr ? KICK_SEP : KICK_ANY;
@@ -619,7 +619,8 @@ struct BatchWork {
     FastDiv fbpi;
 };
 
-template <typename T, int MODE, int N, int E, int R0, int R1, int R2>
+// FORM: the kick of every instance (between-steps pass), KICK_ANY: of each its own.
+template <typename T, int MODE, int N, int E, int R0, int R1, int R2, int FORM = KICK_ANY>
 __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MINB)
     xbatch_kernel(const PassArgs<T>* __restrict__ args, const BatchWork w) {
     using XS = XShape<T, N, E>;
@@ -635,7 +636,7 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
         const uint32_t inst = fdiv(t, w.fbpi);
         const PassArgs<T>& a = args[inst];
         const long long tile = (long long)(t - inst * w.bpi);
-        if constexpr (MODE == XM_MID) {  // the common between-steps programs: full kick, separable absorber or none
+        if constexpr (MODE == XM_MID && FORM == KICK_ANY) {
             const int form = kick_form(a);
             if (form == KICK_SEP) {
                 xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_SEP, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
@@ -646,7 +647,7 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
                 continue;
             }
         }
-        xpass2_body<T, MODE, N, E, R0, R1, R2, KICK_ANY, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
+        xpass2_body<T, MODE, N, E, R0, R1, R2, FORM, true>(a, tile, xb, tw, TW::lo_of(tw), vt);
     }
 }
 
@@ -665,7 +666,7 @@ constexpr size_t xstage_smem() {
            (size_t)N * sizeof(double);
 }
 
-template <typename T, int N, int E, int R0, int R1, int R2>
+template <typename T, int KICK, int N, int E, int R0, int R1, int R2>
 __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MINB)
     xstage_kernel(const __grid_constant__ PassArgs<T> a, const uint32_t tiles) {
     using XS = XShape<T, N, E>;
@@ -677,19 +678,11 @@ __global__ void __launch_bounds__(XShape<T, N, E>::NW * 32, XShape<T, N, E>::MIN
     double* mrow = reinterpret_cast<double*>(vt + (size_t)XS::NW * XS::LPW * XS::RPITCH);
     TW::load(tw, a.stw, a.stwl);  // a handle's constant table: no need to wait for the previous pass
     pdl_wait();
-    if (a.tb.maskfull == nullptr && a.tb.mask1[0] != nullptr)
+    if constexpr (KICK == KICK_SEP)
         for (int i = threadIdx.x; i < N; i += blockDim.x) mrow[i] = a.tb.mask1[0][i];
     __syncthreads();
-    const int form = kick_form(a);
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const long long tile = (long long)t;
-        if (form == KICK_SEP)
-            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_SEP, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
-        else if (form == KICK_PLAIN)
-            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_PLAIN, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
-        else
-            xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK_ANY, true, true>(a, tile, xb, tw, TW::lo_of(tw), vt, mrow);
-    }
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x)
+        xpass2_body<T, XM_MID, N, E, R0, R1, R2, KICK, true, true>(a, (long long)t, xb, tw, TW::lo_of(tw), vt, mrow);
 }
 
 // Dynamic shared memory of xbatch_kernel: stage twiddles, then NW * LPW table

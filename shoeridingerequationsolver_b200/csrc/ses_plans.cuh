@@ -55,8 +55,8 @@ struct PlanEntry {
     std::vector<SVar> sv;
     // the between-steps contiguous pass of one field on staged rows (xstage_kernel)
     using XStage = void (*)(const PassArgs<T>, uint32_t);
-    XStage xs = nullptr;
-    int xs_bps = 0;
+    XStage xs[3] = {nullptr, nullptr, nullptr};  // by KickForm
+    int xs_bps[3] = {0, 0, 0};
     size_t xssm = 0;
     // default variants (a pipelined variant's index, -1 the register path, x: kXStaged),
     // as measured: the contiguous pass between steps, the other contiguous passes (first
@@ -70,6 +70,8 @@ struct PlanEntry {
     // batched kernels (many fields of this length per launch), by mode
     using XBatch = void (*)(const PassArgs<T>*, const BatchWork);
     XBatch xb[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    XBatch xbf[3] = {nullptr, nullptr, nullptr};  // between steps, by the KickForm of every instance
+    int xbf_bps[3] = {0, 0, 0};
     XBatch sb[kSModes] = {};
     int xb_bps[7] = {0, 0, 0, 0, 0, 0, 0};  // resident CTAs per SM
     int sb_bps[kSModes] = {};
@@ -119,15 +121,28 @@ PlanEntry<T> make_plan_entry() {
     p.sb[SM_TW_MID] = sbatch_kernel<T, SM_TW_MID, N, E, R0, R1, R2, LS>;
     p.sb[SM_TW_END] = sbatch_kernel<T, SM_TW_END, N, E, R0, R1, R2, LS>;
     p.xssm = xstage_smem<T, N, E, R0, R1, R2>();
-    p.xs = xstage_kernel<T, N, E, R0, R1, R2>;
-    allow_smem(p.xs, (int)p.xssm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps, p.xs, p.xw * 32, p.xssm, cudaOccupancyDefault);
+    p.xs[KICK_ANY] = xstage_kernel<T, KICK_ANY, N, E, R0, R1, R2>;
+    p.xs[KICK_SEP] = xstage_kernel<T, KICK_SEP, N, E, R0, R1, R2>;
+    p.xs[KICK_PLAIN] = xstage_kernel<T, KICK_PLAIN, N, E, R0, R1, R2>;
+    for (int k = 0; k < 3; ++k) {
+        allow_smem(p.xs[k], (int)p.xssm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xs_bps[k], p.xs[k], p.xw * 32, p.xssm,
+                                                              cudaOccupancyDefault);
+    }
     for (int m = 0; m < 7; ++m)
         if (p.xb[m]) {
             allow_smem(p.xb[m], (int)p.xbsm);
             cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xb_bps[m], p.xb[m], p.xw * 32, p.xbsm,
                                                                   cudaOccupancyDefault);
         }
+    p.xbf[KICK_ANY] = p.xb[XM_MID];
+    p.xbf[KICK_SEP] = xbatch_kernel<T, XM_MID, N, E, R0, R1, R2, KICK_SEP>;
+    p.xbf[KICK_PLAIN] = xbatch_kernel<T, XM_MID, N, E, R0, R1, R2, KICK_PLAIN>;
+    for (int k = 0; k < 3; ++k) {
+        allow_smem(p.xbf[k], (int)p.xbsm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(&p.xbf_bps[k], p.xbf[k], p.xw * 32, p.xbsm,
+                                                              cudaOccupancyDefault);
+    }
     for (int m = 0; m < kSModes; ++m)
         if (p.sb[m]) {
             allow_smem(p.sb[m], smem + (int)p.twb);

@@ -72,6 +72,45 @@ def test_first_and_last_x_passes(ses, nx, prec, fed):
     op.close()
 
 
+@pytest.mark.parametrize("nx,prec", [(64, "c64"), (96, "c64"), (128, "c64"), (160, "c64"), (256, "c64"), (64, "c128"),
+                                     (128, "c128")])
+def test_batches_split_into_calls_and_mixed_absorbers(ses, oracle, nx, prec):
+    """Members without an absorber, with a separable one and with a full one: all of a class
+    alike, and mixed."""
+    dims = (nx, 32, 32)
+    g, V, psi = scene(ses, dims)
+    profiles = [np.linspace(0.97, 1.0, d) for d in dims]
+    sep = (profiles[0][None, None, :] * profiles[1][None, :, None] * profiles[2][:, None, None]).reshape(-1)
+    full = np.random.default_rng(1).uniform(0.97, 1.0, g.size())
+    tol = 6e-12 if prec == "c128" else 1e-5
+    want = {m: oracle.step3d(g.box, dims, V, 0.01, psi, 6, mask=v) for m, v in (("n", None), ("s", sep), ("f", full))}
+    for members in ("nn", "ss", "ff", "nsf", "sf"):
+        ops = []
+        for m in members:
+            op = ses.SplitOperator3D(g, V, 0.01, precision=prec)
+            if m == "s":
+                op.set_absorber_separable(*profiles)
+            elif m == "f":
+                op.set_absorber(full)
+            ops.append(op)
+        with ses.Batch(ops) as b:
+            assert "member-by-member" not in b.info(), b.info()
+            first = None
+            for split in ((6,), (1, 1, 1, 3)):
+                for op in ops:
+                    op.upload_state(psi)
+                for k in split:
+                    b.step(k, absorb=True)
+                b.sync()
+                outs = [op.readback() for op in ops]
+                first = first or outs
+                assert all(np.array_equal(a, c) for a, c in zip(first, outs)), members
+        for m, out in zip(members, first):
+            assert rel(out, want[m]) < tol, (members, m)
+        for op in ops:
+            op.close()
+
+
 # ---- defaults by the number of lines ----
 
 # (axis, dims with few lines, dims with more, precision, text of the first, text of the second)
