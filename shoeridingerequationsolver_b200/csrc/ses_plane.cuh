@@ -179,12 +179,10 @@ __device__ __forceinline__ void plane_x(const PassArgs<T>& a, int z, int y0, cx<
             }
         }
         if constexpr (MODE == PL_MID) {
-            if (a.d_mid != DG_NONE) {
 #pragma unroll
-                for (int b = 0; b < EX / RL; ++b)
+            for (int b = 0; b < EX / RL; ++b)
 #pragma unroll
-                    for (int r = 0; r < RL; ++r) tv[b * RL + r] = vtab[row + q + TL * b + r * (NX / RL)];
-            }
+                for (int r = 0; r < RL; ++r) tv[b * RL + r] = vtab[row + q + TL * b + r * (NX / RL)];
             if (kPreMask && mrow) {
 #pragma unroll
                 for (int b = 0; b < EX / RL; ++b)
@@ -211,8 +209,8 @@ __device__ __forceinline__ void plane_x(const PassArgs<T>& a, int z, int y0, cx<
                     a.dst[row + pos] = e;
                 }
         } else {
-            // the two programs of the step as straight-line code
-            if (a.d_mid == DG_FULL && mrow) {
+            // the full kick, the only one between steps, with and without the absorber as straight-line code
+            if (mrow) {
 #pragma unroll
                 for (int b = 0; b < EX / RL; ++b)
 #pragma unroll
@@ -221,19 +219,9 @@ __device__ __forceinline__ void plane_x(const PassArgs<T>& a, int z, int y0, cx<
                         const double m = (kPreMask ? mv[kPreMask ? i : 0] : mrow[q + TL * b + r * (NX / RL)]) * myz;
                         v[i] = apply_diag_tv(cconj(v[i]), DG_FULL, tv[i], 1, m);
                     }
-            } else if (a.d_mid == DG_FULL) {
-#pragma unroll
-                for (int i = 0; i < EX; ++i) v[i] = apply_diag_tv(cconj(v[i]), DG_FULL, tv[i], 0, 1.0);
             } else {
 #pragma unroll
-                for (int b = 0; b < EX / RL; ++b)
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) {
-                        const int i = b * RL + r;
-                        const cx<T> e = cconj(v[i]);
-                        v[i] = apply_diag_tv(e, a.d_mid, a.d_mid != DG_NONE ? tv[i] : e, mrow != nullptr,
-                                             mrow ? mrow[q + TL * b + r * (NX / RL)] * myz : 1.0);
-                    }
+                for (int i = 0; i < EX; ++i) v[i] = apply_diag_tv(cconj(v[i]), DG_FULL, tv[i], 0, 1.0);
             }
             rfft_plan<T, NX, EX, RX0, RX1, RX2, true, PK>(v, q, twx, twx, xw);
 #pragma unroll
