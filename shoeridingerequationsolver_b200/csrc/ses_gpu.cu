@@ -1292,18 +1292,24 @@ bool select_plane(ses_solver* h, int cs) {
 
 // Default step form of a grid with plane passes, from B200 measurements of
 // single-handle n^3 steps with an absorber (us per step: four axis passes / plane on
-// 1 CTA / on a cluster of 2 / of 4): complex64 32: 9.6 / 6.5 / 7.7 / --, 48: 10.8 /
-// 8.2 / 9.5 / --, 64: 11.5 / 10.6 / 9.8 / 10.2, 96: 20.8 / 21.6 / 22.2 / 22.1, 128:
-// 37.5 / 32.1 / --; complex128 32: 9.0 / 7.0 / 7.7 / --, 48: 13.4 / 13.1 / 11.8 / --,
-// 64: 12.9 / 13.1 / 11.4 / 11.6.
+// 1 CTA / on a cluster of 2 / of 4): complex64 32: 9.7 / 6.2 / 7.5 / --, 48: 10.2 /
+// 8.0 / 9.3 / --, 64: 11.7 / 10.6 / 9.9 / 10.3, 96: 20.8 / 21.9 / 22.6 / 22.6, 128:
+// 38.1 / 32.7 / --; complex128 32: 9.1 / 7.0 / 7.5 / --, 48: 13.5 / 13.1 / 11.7 / --,
+// 64: 13.2 / 13.2 / 11.6 / 11.9.  complex64 64 and 96 by the number of planes: a cluster of
+// 2 wins while its CTAs find an SM each (64 x 64 x 64; x 96: 11.9 / 12.5 on 1 / 2), and
+// planes of 96 points, whose one CTA is long, win only where they fill their waves
+// (96 x 96 x 64: 17.1 / 20.2 four passes / 1 CTA, x 128: 27.5 / 24.1, x 192: 45.6 / 50.5).
 template <typename T>
 int default_plane_cs(const ses_solver* h) {
     auto planes = handle_planes<T>(h);
     if (planes.empty()) return 0;
-    const int n = h->n[0];
+    const int n = h->n[0], nz = h->n[2];
     int want = 1;
-    if (sizeof(T) == 8 ? n >= 48 : n == 64) want = 2;
-    if (sizeof(T) == 4 && n == 96) want = 0;
+    if (sizeof(T) == 8 ? n >= 48 : n == 64 && 2 * nz <= h->sms) want = 2;
+    if (sizeof(T) == 4 && n == 96) {
+        const int waves = (nz + h->sms - 1) / h->sms;
+        if (waves > 2 || nz < 0.8 * waves * h->sms) want = 0;
+    }
     for (auto* e : planes)
         if (e->cs == want) return want;
     return 0;  // other variants only when the autotuner or SES_PLANE picks them

@@ -145,6 +145,19 @@ def test_defaults_follow_the_number_of_lines(ses, axis, few, more, prec, t_few, 
         op.close()
 
 
+@pytest.mark.parametrize("dims,prec,form", [((64, 64, 64), "c64", "2 CTAs"), ((64, 64, 96), "c64", "1 CTA "),
+                                            ((96, 96, 64), "c64", "four"), ((96, 96, 128), "c64", "1 CTA "),
+                                            ((96, 96, 192), "c64", "four"), ((64, 64, 64), "c128", "2 CTAs")])
+def test_step_form_follows_the_number_of_planes(ses, oracle, dims, prec, form, monkeypatch):
+    monkeypatch.delenv("SES_PLANE")
+    g, V, psi = scene(ses, dims)
+    op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
+    assert form in op.plan_info(), op.plan_info()
+    op.advance(4)
+    assert rel(op.readback(), oracle.step3d(g.box, dims, V, 0.01, psi, 4)) < (4e-12 if prec == "c128" else 1e-5)
+    op.close()
+
+
 # ---- run-time plans with few lines along y or z: tiles of 1, 2 and 4 lines ----
 
 NARROW = [(64, 1536, 1), (5, 1500, 1), (128, 1000, 1), (256, 300, 1), (100, 2048, 1), (256, 4096, 1), (512, 1000, 1),
