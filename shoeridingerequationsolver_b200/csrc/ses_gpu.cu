@@ -295,6 +295,7 @@ struct ses_solver {
     int xsel = -1;                 // between-steps contiguous pass (-1: register path, kXStaged: staged rows, else a variant)
     int xrest = -1;                // pipelined variant of the other contiguous passes (-1: register path); same bits
     int ssel[3] = {-1, -1, -1};    // pipelined strided-pass variant per axis (-1: register path)
+    bool xgiven = false, sgiven[3] = {false, false, false};  // selected by tuning or the environment, not by default
     // two-sweep 3D step (plane pass with the y transforms, then the z pass) when
     // the x-y plane fits in shared memory: the compiled plane pass (nullptr: not
     // available for this grid) and whether steps use it
@@ -1353,7 +1354,13 @@ void default_variants(ses_solver* h) {
 // (Steps of a line make none between them: there a selection is that of the others.)
 void select_x(ses_solver* h, int v) {
     h->xsel = v;
+    h->xgiven = true;
     if (v != kXStaged && (v >= 0 || h->last_axis == 0)) h->xrest = v;
+}
+
+void select_s(ses_solver* h, int axis, int v) {
+    h->ssel[axis] = v;
+    h->sgiven[axis] = true;
 }
 
 // Selections at creation: defaults, cache, then environment overrides SES_XVAR / SES_SVAR / SES_PLANE.
@@ -1366,7 +1373,7 @@ void apply_selection(ses_solver* h) {
         auto it = cache.find(tune_key(h, a));
         if (it == cache.end()) continue;
         if (a == 0) select_x(h, it->second);
-        else h->ssel[a] = it->second;
+        else select_s(h, a, it->second);
     }
     if (has_planes(h)) {  // cached choice, then SES_PLANE (CTAs per plane; 0 = four axis passes)
         auto it = cache.find(plane_tune_key(h));
@@ -1378,7 +1385,8 @@ void apply_selection(ses_solver* h) {
         if (h->xsel < 0) h->xrest = -1;  // the register path in every pass
     }
     if (const char* e = std::getenv("SES_PDL")) h->pdl = std::atoi(e) != 0;
-    if (const char* e = std::getenv("SES_SVAR")) h->ssel[1] = h->ssel[2] = std::atoi(e);
+    if (const char* e = std::getenv("SES_SVAR"))
+        for (int a : {1, 2}) select_s(h, a, std::atoi(e));
 }
 
 // Mean ms of `reps` calls of one() on the handle's stream after 2 untimed calls.
@@ -1463,7 +1471,7 @@ ses_status autotune_impl(ses_solver* h, int flags) {
         if (axis == 0 && h->last_axis > 0) variants.push_back(kXStaged);
         for (int c : variants) {
             if (axis == 0) select_x(h, c);
-            else h->ssel[axis] = c;
+            else select_s(h, axis, c);
             float ms = 0.f;
             SES_TRY(time_axis_pass<T>(h, axis, 5, &ms));
             if (ms < best_ms) {
@@ -1473,7 +1481,7 @@ ses_status autotune_impl(ses_solver* h, int flags) {
         }
         h->xrest = rest;
         if (axis == 0) select_x(h, best);
-        else h->ssel[axis] = best;
+        else select_s(h, axis, best);
         chosen[tune_key(h, axis)] = best;
     }
     const auto planes = handle_planes<T>(h);
@@ -2164,8 +2172,9 @@ bool svar_ok(const BatchClass& c, int q, int k, int buf) {
     return true;
 }
 
-// Variant per class pass: the batch's autotuned choice, else the on-disk cache,
-// else the plan's measured default; -1 = register-path batched kernel.
+// Variant per class pass: the batch's autotuned choice, else the on-disk cache, else
+// what tuning or the environment gave the first member, else the plan's measured
+// default; -1 = register-path batched kernel.
 template <typename T>
 void class_select(const ses_batch_s* b, BatchClass& c) {
     const ses_solver* h0 = c.mem[0];
@@ -2182,13 +2191,14 @@ void class_select(const ses_batch_s* b, BatchClass& c) {
         return fallback;
     };
     // by default the staged rows of the register path, the fastest for every length between steps
-    const int xs = pick(0, -1);
-    const int rest = reinterpret_cast<const PlanEntry<T>*>(h0->pp[0].cp)->xrest;
+    const int xs = pick(0, h0->xgiven ? h0->xsel : -1);
+    const int rest = h0->xgiven ? h0->xrest : reinterpret_cast<const PlanEntry<T>*>(h0->pp[0].cp)->xrest;
     if (xvar_ok<T>(c, xs)) c.xvar = c.xrest = xs;
     else if (xvar_ok<T>(c, rest)) c.xrest = rest;
     for (int q = 0; q < c.nmid; ++q) {
         const auto* e = reinterpret_cast<const PlanEntry<T>*>(h0->pp[c.mid_axis[q]].cp);
-        const int ss = pick(1 + q, !e ? -1 : (c.mid_mode[q] == SM_FUSED ? e->bfdef : e->bsdef));
+        const int def = !e ? -1 : (c.mid_mode[q] == SM_FUSED ? e->bfdef : e->bsdef);
+        const int ss = pick(1 + q, h0->sgiven[c.mid_axis[q]] ? h0->ssel[c.mid_axis[q]] : def);
         if (svar_ok<T>(c, q, ss, 0)) c.svar[q] = ss;
     }
 }
