@@ -1526,11 +1526,15 @@ std::string plan_info_t(const ses_solver* h) {
             if (e->r1 > 1) o << "x" << e->r1;
             if (e->r2 > 1) o << "x" << e->r2;
             o << " E=" << e->e;
-            const int sel = a == 0 ? h->xsel : h->ssel[a];
-            const int nv = a == 0 ? (int)e->xv.size() : (int)e->sv.size();
-            if (h->pipelined && a == 0 && sel == kXStaged) {
+            // the kernel of the steps' pass, as launch() chooses it
+            const bool line = h->last_axis == 0 && !h->long1d;
+            const int sel = a == 0 ? x_choice<T>(h, h->last_axis == 0 || h->long1d ? XM_1D : XM_MID)
+                                   : s_choice<T>(h, a, h->long1d ? SM_TW_MID : (a == h->last_axis ? SM_FUSED : SM_FWD), 0);
+            if (line) {
+                o << " transforms, steps on a run-time plan (" << h->pp[a].g.nst << " stages)";
+            } else if (a == 0 && sel == kXStaged) {
                 o << " staged rows";
-            } else if (!h->pipelined || sel < 0 || sel >= nv) {
+            } else if (sel < 0) {
                 o << " register-path";
             } else if (a == 0) {
                 o << " pipelined warps=" << e->xv[sel].warps << " ring=" << e->xv[sel].nbuf << " (variant "

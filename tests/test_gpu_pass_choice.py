@@ -176,3 +176,29 @@ def test_narrow_tiles(ses, oracle, dims, prec):
     want = np.fft.fftn(psi.reshape(g.shape)).reshape(-1)
     assert rel(op.readback(), want) < (1e-14 if prec == "c128" else 5e-7) * np.log2(g.size())
     op.close()
+
+
+# ---- what plan_info says ----
+
+@pytest.mark.parametrize("prec", ["c64", "c128"])
+def test_plan_info_names_the_kernels_that_run(ses, prec, monkeypatch):
+    g, V, psi = scene(ses, (128, 1, 1))
+    op = ses.SplitOperator3D(g, V, 0.01, precision=prec)  # a line steps on the run-time plan's kernel
+    assert "run-time plan" in op.plan_info() and "staged" not in op.plan_info(), op.plan_info()
+    op.close()
+    line = ses.line_grid(ses.Grid1D(-7.0, 7.0, 24576))  # no cluster: two register-path launches a step
+    op = ses.SplitOperator3D(line, np.zeros(24576), 0.01, precision=prec)
+    assert "staged" not in op.plan_info() and "pipelined" not in op.plan_info(), op.plan_info()
+    op.close()
+    g, V, psi = scene(ses, (100, 128, 72))  # x has no compiled plan, and 100 is no multiple of a y tile's lines
+    op = ses.SplitOperator3D(g, V, 0.01, precision="c64")
+    monkeypatch.setenv("SES_SVAR", "0")
+    forced = ses.SplitOperator3D(g, V, 0.01, precision="c64")
+    assert "register-path" in parts(forced)["y"], forced.plan_info()
+    op.close()
+    forced.close()
+    monkeypatch.setenv("SES_PIPELINED", "0")
+    g, V, psi = scene(ses, (128, 128, 72))
+    op = ses.SplitOperator3D(g, V, 0.01, precision=prec)
+    assert "staged" not in op.plan_info() and "pipelined" not in op.plan_info(), op.plan_info()
+    op.close()
