@@ -270,8 +270,9 @@ SES_API ses_status ses_observe_real_noalloc(const ses_grid_desc* grid, ses_preci
  * axis pass of a step is ONE launch per class whose CTAs walk instance x
  * line tiles.  Classes run concurrently on their own streams; interior steps
  * are CUDA graphs.  Every member keeps its own field, potential table, axis
- * tables, dt, mass and absorber, and computes exactly what ses_gpu_step would
- * with the same step batching.  Shapes without batched kernels step member by
+ * tables, dt, mass and absorber, and computes what ses_gpu_step would, the same
+ * bits alone in a batch and in any mix (outside a batch the step may take another
+ * form or plan -- two sweeps, a line's run-time plan -- which agrees to rounding).  Shapes without batched kernels step member by
  * member.  A member's stream is the batch's stream while it belongs to it;
  * calls on a member (observe, read_psi, ...) stay valid and are ordered after
  * the batch's queued steps.  Destroying a member removes it first.  A batch

@@ -197,7 +197,7 @@ bool plan_pass(int n, int esize, bool strided, long long nlines, PassPlan& pp, s
     while (L > 1 && L / 2 >= nlines) L /= 2;
     // Fewer tiles than SMs: narrower ones, down to a line, while that puts more SMs to work
     // or (rows of 32 bytes left) takes a second butterfly off a thread.  us a step, rows of
-    // 64 bytes -> this, complex64: 64 x 1536 33.0 -> 15.5, 256 x 1000 30.2 -> 15.7.
+    // 64 bytes -> this, complex64: 64 x 1536 33.0 -> 14.8, 256 x 1000 30.2 -> 14.2.
     while (strided && L > 1 && (nlines + L - 1) / L < 148 && L / 2 * widest >= 32 &&
            (2 * ((nlines + L - 1) / L) <= 148 || (L * widest > kLineThreads && L / 2 * esize >= 32)))
         L /= 2;
@@ -275,7 +275,6 @@ struct ses_solver {
 
     double* partials = nullptr;    // per-CTA rows of real-space sums
     double* kpartials = nullptr;   // per-CTA rows of k-space sums (the reduction passes' partials)
-    size_t partial_rows = 0;
     double* dsums = nullptr;
     double* hsums = nullptr;  // pinned
 
@@ -1838,7 +1837,6 @@ ses_status create_impl(const ses_grid_desc* grid, ses_precision prec, double dt,
     // scratch: the k-space copy for observables, and the staging area for
     // complex128 halves on C64 upload/readback ((N+1)/2 * 16 B <= N*8 + 16 B)
     if ((st = dalloc(h, &h->scratch, N * h->esize + 16)) != SES_OK) return bail(st);
-    h->partial_rows = rows;
     if ((st = dalloc(h, (void**)&h->partials, kObsBlocks * kRedR * sizeof(double))) != SES_OK) return bail(st);
     if ((st = dalloc(h, (void**)&h->kpartials, rows * kRedK * sizeof(double))) != SES_OK) return bail(st);
     if ((st = dalloc(h, (void**)&h->dsums, 32 * sizeof(double))) != SES_OK) return bail(st);

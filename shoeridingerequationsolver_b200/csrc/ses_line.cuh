@@ -14,7 +14,8 @@
 //
 // What bounds it: latency and instruction issue on fields in L2, HBM from about
 // 100 MB on.  A tile is sized to 256 threads and at most 64 KB of buffers, so that
-// 2 to 4 CTAs per SM cover each other's barriers; radices up to 10 run in a kernel
+// 2 to 4 CTAs per SM cover each other's barriers (strided tiles keep rows of 64 bytes up to
+// 200 KB of buffers: one CTA per SM for lines above 512 points); radices up to 10 run in a kernel
 // of their own with 64 registers a thread in complex64.  Against the kernels this
 // replaces (radices to 8, one to three more stages, two barriers each, twiddles
 // gathered from one table): 120x100x90 complex128 step 190 -> 57 us, a 1024-point

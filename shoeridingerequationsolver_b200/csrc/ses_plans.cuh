@@ -189,9 +189,9 @@ void add_x_variant(PlanEntry<T>& p) {
         }
     }
     cudaGetLastError();
-    // The passes that apply a kick while they load or store and the plain transform: fed by
-    // TMA wherever it is built, us a step of a one-step call, register path or staged rows
-    // -> variant 0: complex64 256 x 256 31 -> 25, 256^3 539 -> 385; complex128 31 -> 25, 1078 -> 822.
+    // The passes that apply a kick while they load or store, and the plain transform of few
+    // lines: fed by TMA wherever it is built.  us, a one-step call on staged rows -> on
+    // variant 0: complex64 256^3 448 -> 296; complex128 256^3 968 -> 568, 256 x 256 30 -> 22.
     p.xrest = 0;
     p.xv.push_back(v);
 }

@@ -1,9 +1,9 @@
 // Compiled plans with radix-3/5 factors: 48 = 12x4 (complex128: 4x4x3), 96 =
 // 6x4x4 (complex64 strided passes: 12x8), 160 = 10x4x4 (complex64 strided
 // passes: 20x8); radix 6, 10, 12 and 20 are prime-factor butterflies.
-// Pipelined complex64 variants.  Contiguous passes of one field: the register path, which
-// covers a single grid's few tiles better than the persistent staged rows (n^3, us: 96 12.1
-// against 14.3, 160 32.9 against 34.9, complex128 160 46.9 against 58.8).
+// Pipelined complex64 variants.  Between steps, contiguous passes of one field: the register
+// path, which covers a single grid's few tiles better than the persistent staged rows (n^3,
+// us: 96 12.1 against 14.3, 160 32.9 against 34.9, complex128 160 46.9 against 58.8).
 #include "ses_plans.cuh"
 
 namespace sesk {

@@ -49,7 +49,7 @@ X_VARIANTS = [(32, "c64", False), (48, "c64", False), (64, "c64", True), (96, "c
 @pytest.mark.parametrize("nx,prec,fed", X_VARIANTS)
 def test_first_and_last_x_passes(ses, nx, prec, fed):
     """They run on the TMA-fed kernel where one is built (a one-step call of 256^3 complex64
-    takes 385 us so, 539 without), and a run split into calls gives the bits of one call."""
+    takes 296 us so, 448 without), and a run split into calls gives the bits of one call."""
     dims = (nx, 32, 25 if nx < 512 else 9)
     g, V, psi = scene(ses, dims)
     op = ses.SplitOperator3D(g, V, 0.01, precision=prec, psi0=psi)
