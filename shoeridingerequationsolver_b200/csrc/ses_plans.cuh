@@ -264,7 +264,9 @@ void set_defaults(PlanEntry<T>& p, int x, int s, int f, int bs, int bf) {
     p.bfdef = bf;
 }
 
-// The strided and fused defaults of passes of at most `lines` lines.
+// The strided and fused defaults of passes of at most `lines` lines.  The figures beside
+// the calls are us a step of a field with that many lines on the pass, the other passes
+// alike: the choice for few lines / the default.
 template <typename T>
 void set_few(PlanEntry<T>& p, long long lines, int s, int f) {
     p.few_lines = lines;
